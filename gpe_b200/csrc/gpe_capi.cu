@@ -37,6 +37,9 @@ cudaError_t launch_stage_tma_f32(int kind, int R, int ty, dim3 grid, cudaStream_
                                  const StageArgs& a);
 cudaError_t launch_stage_tma_f32x(int kind, int R, int ty, dim3 grid, cudaStream_t st, const TmaMaps& m,
                                   const StageArgs& a);
+cudaError_t stage_tma_occupancy_f64(int kind, int R, int ty, int* ctas_per_sm);
+cudaError_t stage_tma_occupancy_f32(int kind, int R, int ty, int* ctas_per_sm);
+cudaError_t stage_tma_occupancy_f32x(int kind, int R, int ty, int* ctas_per_sm);
 }  // namespace gpe
 
 using namespace gpe;
@@ -67,15 +70,15 @@ struct gpe_handle {
   double dx = 0, dy = 0, dz = 0;
   double* part_a = nullptr;  // block partials (energy / first reduction)
   double* part_b = nullptr;  // block partials (norm / errmax)
-  long long npart = 0;       // partials of one stage launch (one per CTA of grid)
-  dim3 norm_grid;            // k_norm's grid: 32 x 8 tiles x z-chunks
+  dim3 norm_grid;            // k_norm's grid: 32 x 8 tiles x z-chunks of zc planes
   long long norm_npart = 0;  // its partials
   double* dres = nullptr;    // [6] finalised reductions
   double* hres = nullptr;    // pinned mirror of dres
   void* staging = nullptr;
   size_t staging_bytes = 0;
-  int zc = 8;
-  dim3 grid;
+  int zc = 8;                // planes per block of k_norm
+  int zck[K_NUM] = {0};      // planes per CTA of each stage kernel the scheme uses
+  int nsm = 148;             // SMs of the device
   std::string err;
   // optional per-kernel timing (gpe_profile): event pairs around launches
   bool prof = false;
@@ -159,7 +162,6 @@ int fail(gpe_handle* h, int code, const std::string& msg) {
 int validate(const gpe_params* p, std::string& why) { return validate_params(p, why); }
 void layout(const gpe_params* p, Geom& g, int& esz) { param_layout(p, g, esz); }
 int nfields(int scheme) { return scheme_fields(scheme); }
-int choose_zc(const Geom& g, int tile_h, int esz) { return default_zc(g, tile_h, esz); }
 bool encode_field_maps(gpe_handle* h, void* base, CUtensorMap* halo, CUtensorMap* pw) {
   return encode_maps(base, h->g, h->esz, h->R, halo, pw, tile_rows(h->tma_ty));
 }
@@ -170,15 +172,59 @@ int field_of(const gpe_handle* h, const void* p) {
   return -1;
 }
 
+// grid of a stage launch: x-y tiles times z-chunks of the kind's length
+dim3 stage_grid(const gpe_handle* h, int kind) {
+  const int th = tile_rows(h->tma_ty), zc = h->zck[kind];
+  return dim3((h->p.nx + 31) / 32, (h->p.ny + th - 1) / th, (h->p.nz + zc - 1) / zc);
+}
+
+// partials of a stage launch, one per CTA
+long long stage_parts(const gpe_handle* h, int kind) {
+  const dim3 g = stage_grid(h, kind);
+  return (long long)g.x * g.y * g.z;
+}
+
+// Planes per CTA of every stage kernel the handle launches, chosen by the
+// kernel's CTAs per SM (the Cash-Karp stages with many point-wise inputs hold
+// half as many as the others).
+int choose_chunks(gpe_handle* h, int tile_zc) {
+  std::vector<int> kinds = {K_ENERGY};
+  switch (h->p.scheme) {
+    case GPE_EULER: kinds.insert(kinds.end(), {K_EULER}); break;
+    case GPE_RK2: kinds.insert(kinds.end(), {K_RK2_1, K_RK2_2}); break;
+    case GPE_RK4: kinds.insert(kinds.end(), {K_RK4_1, K_RK4_2, K_RK4_3, K_RK4_4}); break;
+    default: kinds.insert(kinds.end(), {K_CK_1, K_CK_2, K_CK_3, K_CK_4, K_CK_5, K_CK_6});
+  }
+  const int th = tile_rows(h->tma_ty);
+  const long long tiles = (long long)((h->p.nx + 31) / 32) * ((h->p.ny + th - 1) / th);
+  for (int k : kinds) {
+    if (tile_zc > 0) {
+      h->zck[k] = std::min(tile_zc, h->p.nz);
+    } else if (!h->use_tma) {
+      h->zck[k] = default_zc(h->g, th, h->esz);
+    } else {
+      int per = 0;
+      cudaError_t e = h->cmode == CM_F64   ? stage_tma_occupancy_f64(k, h->R, h->tma_ty, &per)
+                      : h->cmode == CM_F32 ? stage_tma_occupancy_f32(k, h->R, h->tma_ty, &per)
+                                           : stage_tma_occupancy_f32x(k, h->R, h->tma_ty, &per);
+      CU(h, e);
+      h->zck[k] = balanced_zc(h->g, h->esz, h->R, tiles, (long long)h->nsm * std::max(per, 1));
+    }
+  }
+  return GPE_OK;
+}
+
 cudaError_t launch_raw(gpe_handle* h, int kind, const StageArgs& a_in) {
   StageArgs a = a_in;
   a.status = h->status;
+  a.zc = h->zck[kind];
+  const dim3 grid = stage_grid(h, kind);
   set_f32_constants(a);
   if (!h->use_tma) {
     switch (h->cmode) {
-      case CM_F64: return launch_stage_f64(kind, h->R, 8, h->grid, h->st, a);
-      case CM_F32: return launch_stage_f32(kind, h->R, 8, h->grid, h->st, a);
-      default: return launch_stage_f32x(kind, h->R, 8, h->grid, h->st, a);
+      case CM_F64: return launch_stage_f64(kind, h->R, 8, grid, h->st, a);
+      case CM_F32: return launch_stage_f32(kind, h->R, 8, grid, h->st, a);
+      default: return launch_stage_f32x(kind, h->R, 8, grid, h->st, a);
     }
   }
   TmaMaps m;
@@ -201,9 +247,9 @@ cudaError_t launch_raw(gpe_handle* h, int kind, const StageArgs& a_in) {
     m.pw[t] = h->map_pw[f];
   }
   switch (h->cmode) {
-    case CM_F64: return launch_stage_tma_f64(kind, h->R, h->tma_ty, h->grid, h->st, m, a);
-    case CM_F32: return launch_stage_tma_f32(kind, h->R, h->tma_ty, h->grid, h->st, m, a);
-    default: return launch_stage_tma_f32x(kind, h->R, h->tma_ty, h->grid, h->st, m, a);
+    case CM_F64: return launch_stage_tma_f64(kind, h->R, h->tma_ty, grid, h->st, m, a);
+    case CM_F32: return launch_stage_tma_f32(kind, h->R, h->tma_ty, grid, h->st, m, a);
+    default: return launch_stage_tma_f32x(kind, h->R, h->tma_ty, grid, h->st, m, a);
   }
 }
 
@@ -327,8 +373,8 @@ StageArgs base_args(gpe_handle* h) {
   return a;
 }
 
-int finalize_into(gpe_handle* h, const double* part, int slot, long long nparts = -1) {
-  k_finalize<<<1, 256, 0, h->st>>>(part, nparts < 0 ? h->npart : nparts, h->dres + 3 * slot);
+int finalize_into(gpe_handle* h, const double* part, int slot, long long nparts) {
+  k_finalize<<<1, 256, 0, h->st>>>(part, nparts, h->dres + 3 * slot);
   CU(h, cudaGetLastError());
   return GPE_OK;
 }
@@ -391,7 +437,7 @@ int enqueue_fixed_step(gpe_handle* h, double dr, double di, bool energy, bool no
     a.want_energy = energy;
     a.partials = energy ? h->part_a : nullptr;
     CU(h, launch(h, K_RK4_1, a));
-    if (energy && finalize_into(h, h->part_a, 0)) return GPE_ERR_CUDA;
+    if (energy && finalize_into(h, h->part_a, 0, stage_parts(h, K_RK4_1))) return GPE_ERR_CUDA;
     a.want_energy = 0;
     a.partials = nullptr;
     // s2: k2 = f(A); B = psi + dt/2 k2; Q = (psi + A) + dt k2
@@ -409,7 +455,7 @@ int enqueue_fixed_step(gpe_handle* h, double dr, double di, bool energy, bool no
     a.want_norm = norm;
     a.partials = norm ? h->part_b : nullptr;
     CU(h, launch(h, K_RK4_4, a));
-    if (norm && finalize_into(h, h->part_b, 1)) return GPE_ERR_CUDA;
+    if (norm && finalize_into(h, h->part_b, 1, stage_parts(h, K_RK4_4))) return GPE_ERR_CUDA;
     return GPE_OK;
   }
   if (sc == GPE_RK2) {
@@ -419,14 +465,14 @@ int enqueue_fixed_step(gpe_handle* h, double dr, double di, bool energy, bool no
     a.want_energy = energy;
     a.partials = energy ? h->part_a : nullptr;
     CU(h, launch(h, K_RK2_1, a));
-    if (energy && finalize_into(h, h->part_a, 0)) return GPE_ERR_CUDA;
+    if (energy && finalize_into(h, h->part_a, 0, stage_parts(h, K_RK2_1))) return GPE_ERR_CUDA;
     a.want_energy = 0;
     a.in = A; a.psi = psi; a.out = psi;
     a.cf_r[0] = dr; a.cf_i[0] = di;
     a.want_norm = norm;
     a.partials = norm ? h->part_b : nullptr;
     CU(h, launch(h, K_RK2_2, a));
-    if (norm && finalize_into(h, h->part_b, 1)) return GPE_ERR_CUDA;
+    if (norm && finalize_into(h, h->part_b, 1, stage_parts(h, K_RK2_2))) return GPE_ERR_CUDA;
     return GPE_OK;
   }
   // Euler: new = old + dt f(old), written into the other buffer
@@ -438,11 +484,11 @@ int enqueue_fixed_step(gpe_handle* h, double dr, double di, bool energy, bool no
   if (energy && !norm) {
     a.partials = h->part_a;
     CU(h, launch(h, K_EULER, a));
-    if (finalize_into(h, h->part_a, 0)) return GPE_ERR_CUDA;
+    if (finalize_into(h, h->part_a, 0, stage_parts(h, K_EULER))) return GPE_ERR_CUDA;
   } else {
     a.partials = norm ? h->part_b : nullptr;
     CU(h, launch(h, K_EULER, a));
-    if (norm && finalize_into(h, h->part_b, 1)) return GPE_ERR_CUDA;
+    if (norm && finalize_into(h, h->part_b, 1, stage_parts(h, K_EULER))) return GPE_ERR_CUDA;
     // one kernel produced both sums: move the energy into its slot
     if (energy) CU(h, cudaMemcpyAsync(h->dres + 1, h->dres + 4, sizeof(double), cudaMemcpyDeviceToDevice, h->st));
   }
@@ -491,9 +537,9 @@ int rk45_step(gpe_handle* h, gpe_step_info* io, bool energy, bool norm) {
       a.want_energy = (m == 0 && energy && first);
       a.partials = (m == 5) ? h->part_b : (a.want_energy ? h->part_a : nullptr);
       CU(h, launch(h, K_CK_1 + m, a));
-      if (a.want_energy && finalize_into(h, h->part_a, 0)) return GPE_ERR_CUDA;
+      if (a.want_energy && finalize_into(h, h->part_a, 0, stage_parts(h, K_CK_1))) return GPE_ERR_CUDA;
     }
-    if (finalize_into(h, h->part_b, 1)) return GPE_ERR_CUDA;
+    if (finalize_into(h, h->part_b, 1, stage_parts(h, K_CK_6))) return GPE_ERR_CUDA;
     if (int rc = fetch_results(h)) return rc;
     first = false;
     errmax = h->hres[5] / eps;
@@ -688,18 +734,19 @@ int create_impl(const gpe_params* p, const SlabSpec* sp, gpe_handle** out) {
     if (v == TILE_32x8_ROW1 || v == TILE_32x8_ROW2 || (h->cmode == CM_F32 && h->use_tma && tile_is_pair(v)))
       h->tma_ty = v;
   }
-  const int th = tile_rows(h->tma_ty);
-  h->zc = p->tile_zc > 0 ? std::min(p->tile_zc, pl.nz) : choose_zc(h->g, th, h->esz);
-  h->grid = dim3((pl.nx + 31) / 32, (pl.ny + th - 1) / th, (pl.nz + h->zc - 1) / h->zc);
-  h->npart = (long long)h->grid.x * h->grid.y * h->grid.z;
+  h->nsm = prop.multiProcessorCount;
+  h->zc = p->tile_zc > 0 ? std::min(p->tile_zc, pl.nz) : default_zc(h->g, tile_rows(h->tma_ty), h->esz);
   h->norm_grid = dim3((pl.nx + 31) / 32, (pl.ny + 7) / 8, (pl.nz + h->zc - 1) / h->zc);
   h->norm_npart = (long long)h->norm_grid.x * h->norm_grid.y * h->norm_grid.z;
-  const long long npart_alloc = std::max(h->npart, h->norm_npart);
   auto bail = [&](int rc) {
     std::string m = h->err;
     gpe_destroy(h);
     return fail(nullptr, rc, m);
   };
+  if (int rc = choose_chunks(h, p->tile_zc)) return bail(rc);
+  long long npart_alloc = h->norm_npart;
+  for (int k = 0; k < K_NUM; ++k)
+    if (h->zck[k]) npart_alloc = std::max(npart_alloc, stage_parts(h, k));
   if (sp && sp->hub) {
     h->hub = sp->hub;
     h->st = sp->hub->st;
@@ -1121,7 +1168,7 @@ int gpe_energy(gpe_handle* h, double* energy) {
   a.want_energy = 1;
   a.partials = h->part_a;
   CU(h, launch(h, K_ENERGY, a));
-  if (int rc = finalize_into(h, h->part_a, 0)) return rc;
+  if (int rc = finalize_into(h, h->part_a, 0, stage_parts(h, K_ENERGY))) return rc;
   if (int rc = fetch_results(h)) return rc;
   *energy = ((h->hres[1] * h->dx) * h->dy) * h->dz;
   return GPE_OK;

@@ -56,18 +56,48 @@ int scheme_fields(int scheme) {
   }
 }
 
-// z planes per block: enough blocks for several waves on 148 SMs
-int default_zc(const Geom& g, int tile_h, int esz) {
-  if (const char* e = getenv("GPE_ZC")) {
-    int v = atoi(e);
-    if (v > 0) return std::min(v, g.nz);
+// GPE_ZC: planes per CTA asked for by name, 0 = none
+static int zc_from_env(int nz) {
+  const char* e = getenv("GPE_ZC");
+  const int v = e ? atoi(e) : 0;
+  return v > 0 ? std::min(v, nz) : 0;
+}
+
+// A launch takes as many rounds as its CTAs need of the device's slots, and a
+// CTA as long as its planes plus what its queue fill and halo planes cost (1
+// plane for R = 1, 6 for R = 2).  Where the launch is one or two rounds the
+// chunk that just fills them is best by a wide margin: RK4, 96^3 complex128
+// order 4 (592 slots) takes 43.3 us a step with 576 CTAs of 6 planes, 55.5
+// with 864 of 4 and 50.6 with 360 of 10; 131 x 97 x 115: 75.7 (585 CTAs of 13
+// planes) against 85.7 with 1105 of 7.  With more rounds their ends overlap:
+// the broken round counts as a whole one less and less (half per round), and
+// equal costs go to the shorter chunk, at most 24 (complex128) or 20
+// (complex64) planes -- 256^3 complex128: 20 and 24 planes 573, 16: 579, 29:
+// 577, 32: 598 us.  Over 77 shapes from 16^3 to 256^3, both orders and
+// storages, the choice is within 0.6 % of the best chunk on average (7 % at
+// worst) and 15 % faster than a fixed target of 8 CTAs per SM.
+int balanced_zc(const Geom& g, int esz, int R, long long tiles, long long slots) {
+  if (const int v = zc_from_env(g.nz)) return v;
+  const double lead = 5 * R - 4;
+  const int zmax = std::min(g.nz, esz >= 16 ? 24 : 20);
+  int best = 1;
+  double best_cost = 0.0;
+  for (int z = 1; z <= zmax; ++z) {
+    const double x = (double)(tiles * ((g.nz + z - 1) / z)) / (double)slots, whole = ceil(x);
+    const double rounds = x <= 1.0 ? 1.0 : x + 0.3 + (whole - x - 0.3) * pow(0.5, whole - 1.0);
+    const double cost = rounds * (z + lead) * (1.0 + 0.004 * z);
+    if (z == 1 || cost < best_cost) {
+      best = z;
+      best_cost = cost;
+    }
   }
-  // at most 24 planes per CTA for complex128 sites (32x8 tiles) and 20 for
-  // complex64 (32x16 two-sites-per-thread tiles): at 256^3, sweeps of
-  // 16..43 planes give these the best rates (complex128: 24 is +0.7 % over
-  // 20 and 29, +3 % over 32; complex64: 20 is +1 % over 29, +2.4 % over 16,
-  // +3.4 % over 24); small grids use fewer so that every SM gets several
-  // CTAs.
+  return best;
+}
+
+// z planes per block: enough blocks for several waves on 148 SMs (the norm
+// kernel and k_stage)
+int default_zc(const Geom& g, int tile_h, int esz) {
+  if (const int v = zc_from_env(g.nz)) return v;
   const long long bxy = (long long)((g.nx + 31) / 32) * ((g.ny + tile_h - 1) / tile_h);
   const long long target = 148LL * 8;
   const long long cap = esz >= 16 ? 24 : 20;

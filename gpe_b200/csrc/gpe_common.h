@@ -22,7 +22,10 @@ void param_layout(const gpe_params* p, Geom& g, int& esz);
 long long padded_elems(const Geom& g);
 // fields a scheme keeps per solve
 int scheme_fields(int scheme);
-// z planes per CTA / work item
+// z planes per CTA of a stage launch over `tiles` x-y tiles when `slots` CTAs
+// of the kernel run at once on the device
+int balanced_zc(const Geom& g, int esz, int R, long long tiles, long long slots);
+// z planes per block of the norm kernel and k_stage
 int default_zc(const Geom& g, int tile_h = 8, int esz = 16);
 // tensor maps of one field: halo'd stencil box and point-wise box of a
 // 32 x tile_h tile

@@ -44,28 +44,37 @@ static cudaError_t launch_kind(int kind, dim3 grid, cudaStream_t st, const Stage
   return cudaGetLastError();
 }
 
-template <class S, class C, int R, int K, int TY, int PY>
-static cudaError_t launch_tma_one(dim3 grid, cudaStream_t st, const TmaMaps& m, const StageArgs& a) {
-  using LY = TmaLayout<S, R, StageTraits<K>::NPW, TY>;
-  static unsigned long long attr_set = 0;  // per instantiation, one bit per device
+// Opt a stage kernel into its dynamic shared memory, once per device (done is
+// the caller's per-instantiation record, one bit per device).
+template <class F>
+static cudaError_t opt_in_smem(F kernel, uint32_t smem, unsigned long long& done) {
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 64 || !(attr_set & (1ULL << dev))) {
-    cudaError_t e = cudaFuncSetAttribute(k_stage_tma<S, C, R, K, TY, PY>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LY::SMEM);
-    if (e != cudaSuccess) return e;
-    if (dev < 64) attr_set |= 1ULL << dev;
-  }
-  k_stage_tma<S, C, R, K, TY, PY><<<grid, dim3(32, TY / PY), LY::SMEM, st>>>(m, a);
+  if (dev < 64 && (done & (1ULL << dev))) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess && dev < 64) done |= 1ULL << dev;
+  return e;
+}
+
+// A null map pointer asks for the kernel's CTAs per SM (in *occ) instead of a launch.
+template <class S, class C, int R, int K, int TY, int PY>
+static cudaError_t launch_tma_one(dim3 grid, cudaStream_t st, const TmaMaps* m, const StageArgs& a, int* occ) {
+  using LY = TmaLayout<S, R, StageTraits<K>::NPW, TY>;
+  static unsigned long long attr_set = 0;
+  cudaError_t e = opt_in_smem(k_stage_tma<S, C, R, K, TY, PY>, LY::SMEM, attr_set);
+  if (e != cudaSuccess) return e;
+  if (!m) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k_stage_tma<S, C, R, K, TY, PY>, 32 * TY / PY, LY::SMEM);
+  k_stage_tma<S, C, R, K, TY, PY><<<grid, dim3(32, TY / PY), LY::SMEM, st>>>(*m, a);
   return cudaGetLastError();
 }
 
 template <class S, class C, int R, int TY, int PY>
-static cudaError_t launch_tma_kind(int kind, dim3 grid, cudaStream_t st, const TmaMaps& m, const StageArgs& a) {
+static cudaError_t launch_tma_kind(int kind, dim3 grid, cudaStream_t st, const TmaMaps* m, const StageArgs& a,
+                                   int* occ) {
   switch (kind) {
 #define GPE_TCASE(K) \
   case K:            \
-    return launch_tma_one<S, C, R, K, TY, PY>(grid, st, m, a);
+    return launch_tma_one<S, C, R, K, TY, PY>(grid, st, m, a, occ);
     GPE_TCASE(K_EULER)
     GPE_TCASE(K_RK2_1)
     GPE_TCASE(K_RK2_2)
@@ -87,28 +96,24 @@ static cudaError_t launch_tma_kind(int kind, dim3 grid, cudaStream_t st, const T
 }
 
 template <class C, int R, int K, int TY, int PY>
-static cudaError_t launch_tma_pair_one(dim3 grid, cudaStream_t st, const TmaMaps& m, const StageArgs& a) {
+static cudaError_t launch_tma_pair_one(dim3 grid, cudaStream_t st, const TmaMaps* m, const StageArgs& a, int* occ) {
   using LY = TmaLayout<float2, R, StageTraits<K>::NPW, TY>;
-  static unsigned long long attr_set = 0;  // per instantiation, one bit per device
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 64 || !(attr_set & (1ULL << dev))) {
-    cudaError_t e = cudaFuncSetAttribute(k_stage_tma_pair<C, R, K, TY, PY>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LY::SMEM);
-    if (e != cudaSuccess) return e;
-    if (dev < 64) attr_set |= 1ULL << dev;
-  }
-  k_stage_tma_pair<C, R, K, TY, PY><<<grid, dim3(16, TY / PY), LY::SMEM, st>>>(m, a);
+  static unsigned long long attr_set = 0;
+  cudaError_t e = opt_in_smem(k_stage_tma_pair<C, R, K, TY, PY>, LY::SMEM, attr_set);
+  if (e != cudaSuccess) return e;
+  if (!m)
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k_stage_tma_pair<C, R, K, TY, PY>, 16 * TY / PY, LY::SMEM);
+  k_stage_tma_pair<C, R, K, TY, PY><<<grid, dim3(16, TY / PY), LY::SMEM, st>>>(*m, a);
   return cudaGetLastError();
 }
 
 template <class C, int R, int TY, int PY>
-static cudaError_t launch_tma_pair_kind(int kind, dim3 grid, cudaStream_t st, const TmaMaps& m,
-                                        const StageArgs& a) {
+static cudaError_t launch_tma_pair_kind(int kind, dim3 grid, cudaStream_t st, const TmaMaps* m,
+                                        const StageArgs& a, int* occ) {
   switch (kind) {
 #define GPE_PCASE(K) \
   case K:            \
-    return launch_tma_pair_one<C, R, K, TY, PY>(grid, st, m, a);
+    return launch_tma_pair_one<C, R, K, TY, PY>(grid, st, m, a, occ);
     GPE_PCASE(K_EULER)
     GPE_PCASE(K_RK2_1)
     GPE_PCASE(K_RK2_2)
@@ -130,25 +135,25 @@ static cudaError_t launch_tma_pair_kind(int kind, dim3 grid, cudaStream_t st, co
 }
 
 template <class S, class C>
-static cudaError_t launch_stage_tma_impl(int kind, int R, int ty, dim3 grid, cudaStream_t st, const TmaMaps& m,
-                                         const StageArgs& a) {
+static cudaError_t launch_stage_tma_impl(int kind, int R, int ty, dim3 grid, cudaStream_t st, const TmaMaps* m,
+                                         const StageArgs& a, int* occ) {
   // ty is a TileVariant: TILE_32x8_ROW1 / TILE_32x8_ROW2 (any storage), or
   // the pair layouts (complex64 storage with FP32 stencil compute)
   if constexpr (std::is_same<S, float2>::value && std::is_same<C, float>::value) {
     if (ty == TILE_PAIR_32x8) {
-      if (R == 1) return launch_tma_pair_kind<C, 1, 8, 1>(kind, grid, st, m, a);
-      if (R == 2) return launch_tma_pair_kind<C, 2, 8, 1>(kind, grid, st, m, a);
+      if (R == 1) return launch_tma_pair_kind<C, 1, 8, 1>(kind, grid, st, m, a, occ);
+      if (R == 2) return launch_tma_pair_kind<C, 2, 8, 1>(kind, grid, st, m, a, occ);
     } else if (ty == TILE_PAIR_32x16) {
-      if (R == 1) return launch_tma_pair_kind<C, 1, 16, 2>(kind, grid, st, m, a);
-      if (R == 2) return launch_tma_pair_kind<C, 2, 16, 2>(kind, grid, st, m, a);
+      if (R == 1) return launch_tma_pair_kind<C, 1, 16, 2>(kind, grid, st, m, a, occ);
+      if (R == 2) return launch_tma_pair_kind<C, 2, 16, 2>(kind, grid, st, m, a, occ);
     }
   }
   if (ty == 8) {
-    if (R == 1) return launch_tma_kind<S, C, 1, 8, 1>(kind, grid, st, m, a);
-    if (R == 2) return launch_tma_kind<S, C, 2, 8, 1>(kind, grid, st, m, a);
+    if (R == 1) return launch_tma_kind<S, C, 1, 8, 1>(kind, grid, st, m, a, occ);
+    if (R == 2) return launch_tma_kind<S, C, 2, 8, 1>(kind, grid, st, m, a, occ);
   } else if (ty == 4) {
-    if (R == 1) return launch_tma_kind<S, C, 1, 8, 2>(kind, grid, st, m, a);
-    if (R == 2) return launch_tma_kind<S, C, 2, 8, 2>(kind, grid, st, m, a);
+    if (R == 1) return launch_tma_kind<S, C, 1, 8, 2>(kind, grid, st, m, a, occ);
+    if (R == 2) return launch_tma_kind<S, C, 2, 8, 2>(kind, grid, st, m, a, occ);
   }
   return cudaErrorInvalidValue;
 }
@@ -316,7 +321,10 @@ static cudaError_t launch_stage_impl(int kind, int R, int ty, dim3 grid, cudaStr
   }                                                                                                     \
   cudaError_t launch_stage_tma_##TAG(int kind, int R, int ty, dim3 grid, cudaStream_t st, const TmaMaps& m, \
                                      const StageArgs& a) {                                              \
-    return launch_stage_tma_impl<S, C>(kind, R, ty, grid, st, m, a);                                    \
+    return launch_stage_tma_impl<S, C>(kind, R, ty, grid, st, &m, a, nullptr);                          \
+  }                                                                                                     \
+  cudaError_t stage_tma_occupancy_##TAG(int kind, int R, int ty, int* ctas_per_sm) {                    \
+    return launch_stage_tma_impl<S, C>(kind, R, ty, dim3(), nullptr, nullptr, StageArgs(), ctas_per_sm); \
   }                                                                                                     \
   int batch_rows_##TAG(int kind) {                                                                      \
     return (std::is_same<S, float2>::value && std::is_same<C, float>::value && is_rk4_kind(kind))          \
