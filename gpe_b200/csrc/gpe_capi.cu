@@ -200,6 +200,8 @@ int choose_chunks(gpe_handle* h, int tile_zc) {
   for (int k : kinds) {
     if (tile_zc > 0) {
       h->zck[k] = std::min(tile_zc, h->p.nz);
+    } else if (h->tma_ty == TILE_SITE) {
+      h->zck[k] = 1;
     } else if (!h->use_tma) {
       h->zck[k] = default_zc(h->g, th, h->esz);
     } else {
@@ -220,11 +222,12 @@ cudaError_t launch_raw(gpe_handle* h, int kind, const StageArgs& a_in) {
   a.zc = h->zck[kind];
   const dim3 grid = stage_grid(h, kind);
   set_f32_constants(a);
-  if (!h->use_tma) {
+  if (!h->use_tma || h->tma_ty == TILE_SITE) {
+    const int ty = h->tma_ty == TILE_SITE ? TILE_SITE : 8;
     switch (h->cmode) {
-      case CM_F64: return launch_stage_f64(kind, h->R, 8, grid, h->st, a);
-      case CM_F32: return launch_stage_f32(kind, h->R, 8, grid, h->st, a);
-      default: return launch_stage_f32x(kind, h->R, 8, grid, h->st, a);
+      case CM_F64: return launch_stage_f64(kind, h->R, ty, grid, h->st, a);
+      case CM_F32: return launch_stage_f32(kind, h->R, ty, grid, h->st, a);
+      default: return launch_stage_f32x(kind, h->R, ty, grid, h->st, a);
     }
   }
   TmaMaps m;
@@ -731,8 +734,12 @@ int create_impl(const gpe_params* p, const SlabSpec* sp, gpe_handle** out) {
   if (const char* e = getenv("GPE_ROWS_PER_THREAD")) h->tma_ty = atoi(e) == 1 ? TILE_32x8_ROW1 : TILE_32x8_ROW2;
   if (const char* e = getenv("GPE_TILE")) {
     const int v = atoi(e);
-    if (v == TILE_32x8_ROW1 || v == TILE_32x8_ROW2 || (h->cmode == CM_F32 && h->use_tma && tile_is_pair(v)))
+    if (v == TILE_32x8_ROW1 || v == TILE_32x8_ROW2 || v == TILE_SITE ||
+        (h->cmode == CM_F32 && h->use_tma && tile_is_pair(v)))
       h->tma_ty = v;
+  } else if (h->use_tma && p->tile_zc == 0 && !getenv("GPE_ROWS_PER_THREAD") && !getenv("GPE_ZC") &&
+             (long long)((pl.nx + 31) / 32) * ((pl.ny + SITE_TY - 1) / SITE_TY) * pl.nz <= SITE_MAX_BLOCKS) {
+    h->tma_ty = TILE_SITE;  // a small grid, and no layout or chunk asked for
   }
   h->nsm = prop.multiProcessorCount;
   h->zc = p->tile_zc > 0 ? std::min(p->tile_zc, pl.nz) : default_zc(h->g, tile_rows(h->tma_ty), h->esz);

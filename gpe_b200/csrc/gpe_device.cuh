@@ -51,9 +51,20 @@ enum TileVariant : int {
   TILE_32x8_ROW2 = 4,    // 32 x 4 threads, two rows each
   TILE_PAIR_32x8 = 16,   // 16 x 8 threads, one x pair each
   TILE_PAIR_32x16 = 32,  // 16 x 8 threads on a 32 x 16 tile, an x pair in two rows each
+  TILE_SITE = 1,         // 32 x 4 threads, one site each, no march (small grids)
 };
-__host__ __device__ constexpr int tile_rows(int v) { return v == TILE_PAIR_32x16 ? 16 : 8; }
+__host__ __device__ constexpr int tile_rows(int v) { return v == TILE_PAIR_32x16 ? 16 : (v == TILE_SITE ? 4 : 8); }
 __host__ __device__ constexpr bool tile_is_pair(int v) { return v == TILE_PAIR_32x8 || v == TILE_PAIR_32x16; }
+
+// Device status word values (StageArgs::status).  STATUS_EXPIRE_TEST is set
+// by the host only (gpe_test_expire_waits): while it stands, every work item
+// first waits, with a short limit, on a barrier that nothing arrives at, so
+// that the timeout path (abort, drain the issued copies, return) runs; the
+// word keeps the value until the host reads and clears it.
+constexpr int STATUS_OK = 0;
+constexpr int STATUS_WAIT_EXPIRED = 1;
+constexpr int STATUS_EXPIRE_TEST = 2;
+constexpr int EXPIRE_TEST_POLLS = 1 << 10;
 
 // reduction slots in the per-block partials: [norm, energy, errmax]
 enum { RED_NORM = 0, RED_ENERGY = 1, RED_ERR = 2, RED_SLOTS = 3 };
@@ -885,6 +896,65 @@ __global__ void __launch_bounds__(32 * TY) k_stage(const StageArgs a) {
   }
 
   if (a.partials) block_reduce_store<NT>(r_norm, r_en, r_err, a.partials);
+}
+
+// ---------------------------------------------------------------------------
+// The stage kernel of small grids: one thread per site, neighbours read
+// straight through L1.  Grids that leave the SMs with a block or two have no
+// use for a march: a plane of it is a serial chain of a barrier, shared-memory
+// reads and some fifteen dependent FP64 operations (0.6 us measured, and 2R
+// planes of queue fill before the first output), while here every load of a
+// site is issued at once and the launch is as long as one site.  Measured,
+// us per RK4 step, against the march with its best chunk: 32^3 order 4
+// complex128 10.6 / 16.7, 48^3 16.8 / 20.8, 56^3 20.8 / 22.8, 64^3 24.8 /
+// 24.8, 72^3 35.1 / 33.0; complex64 48^3 14.7 / 18.8, 64^3 22.4 / 22.9.
+// ---------------------------------------------------------------------------
+constexpr int SITE_TY = 4;  // rows of a block
+// most blocks the kernel is chosen for (56^3: 1568, 64^3: 2048)
+constexpr long long SITE_MAX_BLOCKS = 1600;
+
+template <class S, class C, int R, int KIND>
+__global__ void __launch_bounds__(32 * SITE_TY) k_stage_site(const __grid_constant__ StageArgs a) {
+  using T = StageTraits<KIND>;
+  constexpr int NPWX = T::NPW > 0 ? T::NPW : 1;
+  const Geom& g = a.g;
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * SITE_TY + threadIdx.y, k = blockIdx.z;
+  const bool active = i < g.nx && j < g.ny;
+  const ColumnConsts<C> cc = column_consts<C>(a, i, j, R, active);
+  const long long px = g.px, pz = g.pz;
+  const long long o = (long long)(k + 2) * pz + (long long)(j + 2) * px + g.xoff + i;
+  double r_norm = 0.0, r_en = 0.0, r_err = 0.0;
+  // timeout test (host-armed only): leave without storing, as the march does
+  if (*(volatile const int*)a.status == STATUS_EXPIRE_TEST) return;
+  if (active) {
+    const S* in = (const S*)a.in + o;
+    Nb<C> n;
+    n.c0 = to_c<C>(ldro(in));
+    n.xm1 = to_c<C>(ldro(in - 1));
+    n.xp1 = to_c<C>(ldro(in + 1));
+    n.ym1 = to_c<C>(ldro(in - px));
+    n.yp1 = to_c<C>(ldro(in + px));
+    n.zm1 = to_c<C>(ldro(in - pz));
+    n.zp1 = to_c<C>(ldro(in + pz));
+    if constexpr (R == 2) {
+      n.xm2 = to_c<C>(ldro(in - 2));
+      n.xp2 = to_c<C>(ldro(in + 2));
+      n.ym2 = to_c<C>(ldro(in - 2 * px));
+      n.yp2 = to_c<C>(ldro(in + 2 * px));
+      n.zm2 = to_c<C>(ldro(in - 2 * pz));
+      n.zp2 = to_c<C>(ldro(in + 2 * pz));
+    } else {
+      n.xm2 = n.xp2 = n.ym2 = n.yp2 = n.zm2 = n.zp2 = cx<C>{0, 0};
+    }
+    S pw[NPWX];
+    int q = 0;
+    if constexpr (T::HAS_PSI) pw[q++] = ldro((const S*)a.psi + o);
+    if constexpr (T::HAS_ACC) pw[q++] = ldro((const S*)a.acc + o);
+#pragma unroll
+    for (int m = 0; m < T::NK; ++m) pw[q++] = ldro((const S*)a.kin[m] + o);
+    site_stage<S, C, R, KIND>(a, n, pw, i, j, k, o, zghost_pos(k, g.nz, R, a.bcs, a.zghost), cc, r_norm, r_en, r_err);
+  }
+  if (a.partials) block_reduce_store<32 * SITE_TY>(r_norm, r_en, r_err, a.partials);
 }
 
 }  // namespace gpe

@@ -304,8 +304,41 @@ static cudaError_t launch_batch_impl(int kind, int R, int grid, cudaStream_t st,
   }
 }
 
+template <class S, class C, int R>
+static cudaError_t launch_site_kind(int kind, dim3 grid, cudaStream_t st, const StageArgs& a) {
+  const dim3 block(32, SITE_TY);
+  switch (kind) {
+#define GPE_SCASE(K) \
+  case K:            \
+    k_stage_site<S, C, R, K><<<grid, block, 0, st>>>(a); \
+    break;
+    GPE_SCASE(K_EULER)
+    GPE_SCASE(K_RK2_1)
+    GPE_SCASE(K_RK2_2)
+    GPE_SCASE(K_RK4_1)
+    GPE_SCASE(K_RK4_2)
+    GPE_SCASE(K_RK4_3)
+    GPE_SCASE(K_RK4_4)
+    GPE_SCASE(K_CK_1)
+    GPE_SCASE(K_CK_2)
+    GPE_SCASE(K_CK_3)
+    GPE_SCASE(K_CK_4)
+    GPE_SCASE(K_CK_5)
+    GPE_SCASE(K_CK_6)
+    GPE_SCASE(K_ENERGY)
+#undef GPE_SCASE
+    default:
+      return cudaErrorInvalidValue;
+  }
+  return cudaGetLastError();
+}
+
 template <class S, class C>
 static cudaError_t launch_stage_impl(int kind, int R, int ty, dim3 grid, cudaStream_t st, const StageArgs& a) {
+  if (ty == TILE_SITE) {
+    if (R == 1) return launch_site_kind<S, C, 1>(kind, grid, st, a);
+    if (R == 2) return launch_site_kind<S, C, 2>(kind, grid, st, a);
+  }
   if (ty != 8) return cudaErrorInvalidValue;
   if (R == 1) return launch_kind<S, C, 1, 8>(kind, grid, st, a);
   if (R == 2) return launch_kind<S, C, 2, 8>(kind, grid, st, a);

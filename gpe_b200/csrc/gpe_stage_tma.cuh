@@ -79,16 +79,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
-// Device status word values (StageArgs::status).  STATUS_EXPIRE_TEST is set
-// by the host only (gpe_test_expire_waits): while it stands, every work item
-// first waits, with a short limit, on a barrier that nothing arrives at, so
-// that the timeout path (abort, drain the issued copies, return) runs; the
-// word keeps the value until the host reads and clears it.
-constexpr int STATUS_OK = 0;
-constexpr int STATUS_WAIT_EXPIRED = 1;
-constexpr int STATUS_EXPIRE_TEST = 2;
-constexpr int EXPIRE_TEST_POLLS = 1 << 10;
-
 // Copy stage arguments from the device table through the read-only path.
 __device__ __forceinline__ StageArgs __ldg_args(const StageArgs* p) {
   StageArgs a;

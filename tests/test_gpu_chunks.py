@@ -49,3 +49,17 @@ def test_states_do_not_depend_on_the_chunks(gpu, shape, storage, scheme, order):
     assert info.norm == pytest.approx(iref.norm, rel=tol)
     assert info.energy == pytest.approx(iref.energy, rel=tol) and e == pytest.approx(eref, rel=tol)
     assert (info.t, info.dt_re, info.errmax) == (iref.t, iref.dt_re, iref.errmax)
+
+
+@pytest.mark.parametrize("eqn", [1, 2, 3])
+@pytest.mark.parametrize("bcs,order", [(1, 4), (1, 2), (2, 4)])
+@pytest.mark.parametrize("storage", ["c128", "c64"])
+def test_small_grid_kernel_equals_the_march(gpu, eqn, bcs, order, storage):
+    # 35 x 22 x 13 is a small grid (one thread per site); any chunk asked for selects the march
+    rp = RunParams(nx=35, ny=22, nz=13, xr=4.25, yr=2.625, zr=1.5, tau=0.001, scheme="rk4", eqn_to_solve=eqn, bcs=bcs,
+                   order=order, Urhs=0.2, diss_amp=0.1 if eqn != 2 else 0.0, storage=storage)
+    rng = np.random.default_rng(eqn + 10 * bcs + order)
+    psi0 = 1.0 + 0.3 * (rng.normal(size=(13, 22, 35)) + 1j * rng.normal(size=(13, 22, 35)))
+    ref, _, _ = run(rp, psi0, 4)
+    out, _, _ = run(rp, psi0, 0)
+    np.testing.assert_array_equal(out, ref)
