@@ -28,15 +28,15 @@
 #include "gpe_slab.h"
 
 namespace gpe {
-cudaError_t launch_stage_f64(int kind, int R, int ty, dim3 grid, cudaStream_t st, const StageArgs& a);
-cudaError_t launch_stage_f32(int kind, int R, int ty, dim3 grid, cudaStream_t st, const StageArgs& a);
-cudaError_t launch_stage_f32x(int kind, int R, int ty, dim3 grid, cudaStream_t st, const StageArgs& a);
+cudaError_t launch_stage_f64(int kind, int R, int ty, dim3 grid, cudaStream_t st, const StageArgs& a, bool dep);
+cudaError_t launch_stage_f32(int kind, int R, int ty, dim3 grid, cudaStream_t st, const StageArgs& a, bool dep);
+cudaError_t launch_stage_f32x(int kind, int R, int ty, dim3 grid, cudaStream_t st, const StageArgs& a, bool dep);
 cudaError_t launch_stage_tma_f64(int kind, int R, int ty, dim3 grid, cudaStream_t st, const TmaMaps& m,
-                                 const StageArgs& a);
+                                 const StageArgs& a, bool dep);
 cudaError_t launch_stage_tma_f32(int kind, int R, int ty, dim3 grid, cudaStream_t st, const TmaMaps& m,
-                                 const StageArgs& a);
+                                 const StageArgs& a, bool dep);
 cudaError_t launch_stage_tma_f32x(int kind, int R, int ty, dim3 grid, cudaStream_t st, const TmaMaps& m,
-                                  const StageArgs& a);
+                                  const StageArgs& a, bool dep);
 cudaError_t stage_tma_occupancy_f64(int kind, int R, int ty, int* ctas_per_sm);
 cudaError_t stage_tma_occupancy_f32(int kind, int R, int ty, int* ctas_per_sm);
 cudaError_t stage_tma_occupancy_f32x(int kind, int R, int ty, int* ctas_per_sm);
@@ -117,8 +117,11 @@ struct gpe_handle {
   bool snap_pending = false;
   // one captured RK4/RK2 step without reductions, replayed by gpe_step
   // (the stage arguments, dt included, are baked into the graph)
-  cudaGraphExec_t step_graph = nullptr;
+  // [0] holds one step, [1] GRAPH_STEPS of them, so that a long run pays a
+  // graph launch and its gap once per GRAPH_STEPS steps
+  cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
   double graph_dr = 0, graph_di = 0;
+  bool capturing = false;  // stage launches become dependents of each other
   // asynchronous state copies (gpe_set_state_async / gpe_get_state_async):
   // host <-> staging transfers on a copy stream, pack/unpack on the solve's
   // stream, ordered by events so transfers overlap the steps around them
@@ -225,9 +228,9 @@ cudaError_t launch_raw(gpe_handle* h, int kind, const StageArgs& a_in) {
   if (!h->use_tma || h->tma_ty == TILE_SITE) {
     const int ty = h->tma_ty == TILE_SITE ? TILE_SITE : 8;
     switch (h->cmode) {
-      case CM_F64: return launch_stage_f64(kind, h->R, ty, grid, h->st, a);
-      case CM_F32: return launch_stage_f32(kind, h->R, ty, grid, h->st, a);
-      default: return launch_stage_f32x(kind, h->R, ty, grid, h->st, a);
+      case CM_F64: return launch_stage_f64(kind, h->R, ty, grid, h->st, a, h->capturing);
+      case CM_F32: return launch_stage_f32(kind, h->R, ty, grid, h->st, a, h->capturing);
+      default: return launch_stage_f32x(kind, h->R, ty, grid, h->st, a, h->capturing);
     }
   }
   TmaMaps m;
@@ -250,9 +253,9 @@ cudaError_t launch_raw(gpe_handle* h, int kind, const StageArgs& a_in) {
     m.pw[t] = h->map_pw[f];
   }
   switch (h->cmode) {
-    case CM_F64: return launch_stage_tma_f64(kind, h->R, h->tma_ty, grid, h->st, m, a);
-    case CM_F32: return launch_stage_tma_f32(kind, h->R, h->tma_ty, grid, h->st, m, a);
-    default: return launch_stage_tma_f32x(kind, h->R, h->tma_ty, grid, h->st, m, a);
+    case CM_F64: return launch_stage_tma_f64(kind, h->R, h->tma_ty, grid, h->st, m, a, h->capturing);
+    case CM_F32: return launch_stage_tma_f32(kind, h->R, h->tma_ty, grid, h->st, m, a, h->capturing);
+    default: return launch_stage_tma_f32x(kind, h->R, h->tma_ty, grid, h->st, m, a, h->capturing);
   }
 }
 
@@ -894,7 +897,8 @@ void gpe_destroy(gpe_handle* h) {
   if (h->status) cudaFree(h->status);
   if (h->fft_work) cudaFree(h->fft_work);
   for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
-  if (h->step_graph) cudaGraphExecDestroy(h->step_graph);
+  for (cudaGraphExec_t g : h->step_graph)
+    if (g) cudaGraphExecDestroy(g);
   for (cudaStream_t c : {h->cp_st, h->cp2_st})
     if (c) {
       cudaStreamSynchronize(c);
@@ -965,28 +969,36 @@ int gpe_get_state_device(gpe_handle* h, void* psi_dev, int32_t dtype) {
   return GPE_OK;
 }
 
-// Graph of one fixed step for the current dt (captured on first use and
-// whenever dt changes).  Only for schemes that keep psi in place.
-static int ensure_step_graph(gpe_handle* h, double dr, double di) {
-  if (h->step_graph && h->graph_dr == dr && h->graph_di == di) return GPE_OK;
-  if (h->step_graph) {
-    cudaGraphExecDestroy(h->step_graph);
-    h->step_graph = nullptr;
+// Graph of one (which = 0) or GRAPH_STEPS (1) fixed steps for the current dt,
+// captured on first use and whenever dt changes.  Only for schemes that keep
+// psi in place.
+constexpr int GRAPH_STEPS = 8;
+static int ensure_step_graph(gpe_handle* h, int which, double dr, double di) {
+  if (h->graph_dr != dr || h->graph_di != di) {
+    for (cudaGraphExec_t& g : h->step_graph) {
+      if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
+    h->graph_dr = dr;
+    h->graph_di = di;
   }
+  if (h->step_graph[which]) return GPE_OK;
   cudaGraph_t g = nullptr;
   CU(h, cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
-  const int rc = enqueue_fixed_step(h, dr, di, false, false);
+  h->capturing = true;
+  int rc = GPE_OK;
+  for (int s = 0; s < (which ? GRAPH_STEPS : 1) && rc == GPE_OK; ++s) rc = enqueue_fixed_step(h, dr, di, false, false);
+  h->capturing = false;
   const cudaError_t e = cudaStreamEndCapture(h->st, &g);
   if (rc != GPE_OK) {
     if (e == cudaSuccess && g) cudaGraphDestroy(g);
     return rc;
   }
   CU(h, e);
-  const cudaError_t ei = cudaGraphInstantiate(&h->step_graph, g, 0);
+  const cudaError_t ei = cudaGraphInstantiate(&h->step_graph[which], g, 0);
   cudaGraphDestroy(g);
+  if (ei != cudaSuccess) h->step_graph[which] = nullptr;
   CU(h, ei);
-  h->graph_dr = dr;
-  h->graph_di = di;
   return GPE_OK;
 }
 
@@ -1018,18 +1030,25 @@ static int step_impl(gpe_handle* h, int64_t nsteps, gpe_step_info* io, bool wait
     // one per stage); the first step of a call runs plainly, so every kernel
     // has been loaded and configured before any capture
     const bool graphs = use_step_graphs(h) && nsteps >= 3;
-    for (int64_t s = 0; s < nsteps; ++s) {
+    for (int64_t s = 0; s < nsteps;) {
       const bool e = want_e && s == 0, n = want_n && s == nsteps - 1;
+      int64_t took = 1;
       if (graphs && s > 0 && !e && !n) {
-        if (int rc = ensure_step_graph(h, dr, di)) return rc;
-        CU(h, cudaGraphLaunch(h->step_graph, h->st));
+        const int64_t left = nsteps - s - (want_n ? 1 : 0);  // steps without reductions
+        const int which = left >= GRAPH_STEPS ? 1 : 0;
+        if (int rc = ensure_step_graph(h, which, dr, di)) return rc;
+        CU(h, cudaGraphLaunch(h->step_graph[which], h->st));
+        if (which) took = GRAPH_STEPS;
       } else if (int rc = enqueue_fixed_step(h, dr, di, e, n)) {
         return rc;
       }
-      io->t = io->t + dr;
-      io->im_t = io->im_t + fabs(di);
-      io->p += 1;
-      io->accepted += 1;
+      s += took;
+      for (int64_t q = 0; q < took; ++q) {
+        io->t = io->t + dr;
+        io->im_t = io->im_t + fabs(di);
+      }
+      io->p += took;
+      io->accepted += took;
     }
     if (!wait) return GPE_OK;
     if (int rc = fetch_results(h)) return rc;

@@ -15,6 +15,28 @@ namespace gpe {
 // rows of the 32 x 8 tile owned by each thread of the batched kernel
 constexpr int BATCH_PY = 2;
 
+// Launch a stage kernel, as a dependent of the kernel before it on the stream
+// if dep (programmatic dependent launch).
+template <class... KArgs, class... Args>
+static cudaError_t launch_stage_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                       bool dep, const Args&... args) {
+  if (!dep) {
+    kernel<<<grid, block, smem, st>>>(args...);
+    return cudaGetLastError();
+  }
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, args...);
+}
+
 template <class S, class C, int R, int TY>
 static cudaError_t launch_kind(int kind, dim3 grid, cudaStream_t st, const StageArgs& a) {
   const dim3 block(32, TY);
@@ -58,23 +80,23 @@ static cudaError_t opt_in_smem(F kernel, uint32_t smem, unsigned long long& done
 
 // A null map pointer asks for the kernel's CTAs per SM (in *occ) instead of a launch.
 template <class S, class C, int R, int K, int TY, int PY>
-static cudaError_t launch_tma_one(dim3 grid, cudaStream_t st, const TmaMaps* m, const StageArgs& a, int* occ) {
+static cudaError_t launch_tma_one(dim3 grid, cudaStream_t st, const TmaMaps* m, const StageArgs& a, bool dep,
+                                  int* occ) {
   using LY = TmaLayout<S, R, StageTraits<K>::NPW, TY>;
   static unsigned long long attr_set = 0;
   cudaError_t e = opt_in_smem(k_stage_tma<S, C, R, K, TY, PY>, LY::SMEM, attr_set);
   if (e != cudaSuccess) return e;
   if (!m) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k_stage_tma<S, C, R, K, TY, PY>, 32 * TY / PY, LY::SMEM);
-  k_stage_tma<S, C, R, K, TY, PY><<<grid, dim3(32, TY / PY), LY::SMEM, st>>>(*m, a);
-  return cudaGetLastError();
+  return launch_stage_kernel(k_stage_tma<S, C, R, K, TY, PY>, grid, dim3(32, TY / PY), LY::SMEM, st, dep, *m, a);
 }
 
 template <class S, class C, int R, int TY, int PY>
-static cudaError_t launch_tma_kind(int kind, dim3 grid, cudaStream_t st, const TmaMaps* m, const StageArgs& a,
+static cudaError_t launch_tma_kind(int kind, dim3 grid, cudaStream_t st, const TmaMaps* m, const StageArgs& a, bool dep,
                                    int* occ) {
   switch (kind) {
 #define GPE_TCASE(K) \
   case K:            \
-    return launch_tma_one<S, C, R, K, TY, PY>(grid, st, m, a, occ);
+    return launch_tma_one<S, C, R, K, TY, PY>(grid, st, m, a, dep, occ);
     GPE_TCASE(K_EULER)
     GPE_TCASE(K_RK2_1)
     GPE_TCASE(K_RK2_2)
@@ -96,24 +118,24 @@ static cudaError_t launch_tma_kind(int kind, dim3 grid, cudaStream_t st, const T
 }
 
 template <class C, int R, int K, int TY, int PY>
-static cudaError_t launch_tma_pair_one(dim3 grid, cudaStream_t st, const TmaMaps* m, const StageArgs& a, int* occ) {
+static cudaError_t launch_tma_pair_one(dim3 grid, cudaStream_t st, const TmaMaps* m, const StageArgs& a, bool dep,
+                                  int* occ) {
   using LY = TmaLayout<float2, R, StageTraits<K>::NPW, TY>;
   static unsigned long long attr_set = 0;
   cudaError_t e = opt_in_smem(k_stage_tma_pair<C, R, K, TY, PY>, LY::SMEM, attr_set);
   if (e != cudaSuccess) return e;
   if (!m)
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k_stage_tma_pair<C, R, K, TY, PY>, 16 * TY / PY, LY::SMEM);
-  k_stage_tma_pair<C, R, K, TY, PY><<<grid, dim3(16, TY / PY), LY::SMEM, st>>>(*m, a);
-  return cudaGetLastError();
+  return launch_stage_kernel(k_stage_tma_pair<C, R, K, TY, PY>, grid, dim3(16, TY / PY), LY::SMEM, st, dep, *m, a);
 }
 
 template <class C, int R, int TY, int PY>
 static cudaError_t launch_tma_pair_kind(int kind, dim3 grid, cudaStream_t st, const TmaMaps* m,
-                                        const StageArgs& a, int* occ) {
+                                        const StageArgs& a, bool dep, int* occ) {
   switch (kind) {
 #define GPE_PCASE(K) \
   case K:            \
-    return launch_tma_pair_one<C, R, K, TY, PY>(grid, st, m, a, occ);
+    return launch_tma_pair_one<C, R, K, TY, PY>(grid, st, m, a, dep, occ);
     GPE_PCASE(K_EULER)
     GPE_PCASE(K_RK2_1)
     GPE_PCASE(K_RK2_2)
@@ -136,24 +158,24 @@ static cudaError_t launch_tma_pair_kind(int kind, dim3 grid, cudaStream_t st, co
 
 template <class S, class C>
 static cudaError_t launch_stage_tma_impl(int kind, int R, int ty, dim3 grid, cudaStream_t st, const TmaMaps* m,
-                                         const StageArgs& a, int* occ) {
+                                        const StageArgs& a, bool dep, int* occ) {
   // ty is a TileVariant: TILE_32x8_ROW1 / TILE_32x8_ROW2 (any storage), or
   // the pair layouts (complex64 storage with FP32 stencil compute)
   if constexpr (std::is_same<S, float2>::value && std::is_same<C, float>::value) {
     if (ty == TILE_PAIR_32x8) {
-      if (R == 1) return launch_tma_pair_kind<C, 1, 8, 1>(kind, grid, st, m, a, occ);
-      if (R == 2) return launch_tma_pair_kind<C, 2, 8, 1>(kind, grid, st, m, a, occ);
+      if (R == 1) return launch_tma_pair_kind<C, 1, 8, 1>(kind, grid, st, m, a, dep, occ);
+      if (R == 2) return launch_tma_pair_kind<C, 2, 8, 1>(kind, grid, st, m, a, dep, occ);
     } else if (ty == TILE_PAIR_32x16) {
-      if (R == 1) return launch_tma_pair_kind<C, 1, 16, 2>(kind, grid, st, m, a, occ);
-      if (R == 2) return launch_tma_pair_kind<C, 2, 16, 2>(kind, grid, st, m, a, occ);
+      if (R == 1) return launch_tma_pair_kind<C, 1, 16, 2>(kind, grid, st, m, a, dep, occ);
+      if (R == 2) return launch_tma_pair_kind<C, 2, 16, 2>(kind, grid, st, m, a, dep, occ);
     }
   }
   if (ty == 8) {
-    if (R == 1) return launch_tma_kind<S, C, 1, 8, 1>(kind, grid, st, m, a, occ);
-    if (R == 2) return launch_tma_kind<S, C, 2, 8, 1>(kind, grid, st, m, a, occ);
+    if (R == 1) return launch_tma_kind<S, C, 1, 8, 1>(kind, grid, st, m, a, dep, occ);
+    if (R == 2) return launch_tma_kind<S, C, 2, 8, 1>(kind, grid, st, m, a, dep, occ);
   } else if (ty == 4) {
-    if (R == 1) return launch_tma_kind<S, C, 1, 8, 2>(kind, grid, st, m, a, occ);
-    if (R == 2) return launch_tma_kind<S, C, 2, 8, 2>(kind, grid, st, m, a, occ);
+    if (R == 1) return launch_tma_kind<S, C, 1, 8, 2>(kind, grid, st, m, a, dep, occ);
+    if (R == 2) return launch_tma_kind<S, C, 2, 8, 2>(kind, grid, st, m, a, dep, occ);
   }
   return cudaErrorInvalidValue;
 }
@@ -305,13 +327,12 @@ static cudaError_t launch_batch_impl(int kind, int R, int grid, cudaStream_t st,
 }
 
 template <class S, class C, int R>
-static cudaError_t launch_site_kind(int kind, dim3 grid, cudaStream_t st, const StageArgs& a) {
+static cudaError_t launch_site_kind(int kind, dim3 grid, cudaStream_t st, const StageArgs& a, bool dep) {
   const dim3 block(32, SITE_TY);
   switch (kind) {
 #define GPE_SCASE(K) \
   case K:            \
-    k_stage_site<S, C, R, K><<<grid, block, 0, st>>>(a); \
-    break;
+    return launch_stage_kernel(k_stage_site<S, C, R, K>, grid, block, 0, st, dep, a);
     GPE_SCASE(K_EULER)
     GPE_SCASE(K_RK2_1)
     GPE_SCASE(K_RK2_2)
@@ -330,14 +351,14 @@ static cudaError_t launch_site_kind(int kind, dim3 grid, cudaStream_t st, const 
     default:
       return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 template <class S, class C>
-static cudaError_t launch_stage_impl(int kind, int R, int ty, dim3 grid, cudaStream_t st, const StageArgs& a) {
+static cudaError_t launch_stage_impl(int kind, int R, int ty, dim3 grid, cudaStream_t st, const StageArgs& a,
+                                     bool dep) {
   if (ty == TILE_SITE) {
-    if (R == 1) return launch_site_kind<S, C, 1>(kind, grid, st, a);
-    if (R == 2) return launch_site_kind<S, C, 2>(kind, grid, st, a);
+    if (R == 1) return launch_site_kind<S, C, 1>(kind, grid, st, a, dep);
+    if (R == 2) return launch_site_kind<S, C, 2>(kind, grid, st, a, dep);
   }
   if (ty != 8) return cudaErrorInvalidValue;
   if (R == 1) return launch_kind<S, C, 1, 8>(kind, grid, st, a);
@@ -349,15 +370,16 @@ static cudaError_t launch_stage_impl(int kind, int R, int ty, dim3 grid, cudaStr
 
 #define GPE_DEFINE_LAUNCHER(TAG, S, C)                                                                  \
   namespace gpe {                                                                                       \
-  cudaError_t launch_stage_##TAG(int kind, int R, int ty, dim3 grid, cudaStream_t st, const StageArgs& a) { \
-    return launch_stage_impl<S, C>(kind, R, ty, grid, st, a);                                           \
+  cudaError_t launch_stage_##TAG(int kind, int R, int ty, dim3 grid, cudaStream_t st, const StageArgs& a, \
+                                 bool dep) {                                                            \
+    return launch_stage_impl<S, C>(kind, R, ty, grid, st, a, dep);                                      \
   }                                                                                                     \
   cudaError_t launch_stage_tma_##TAG(int kind, int R, int ty, dim3 grid, cudaStream_t st, const TmaMaps& m, \
-                                     const StageArgs& a) {                                              \
-    return launch_stage_tma_impl<S, C>(kind, R, ty, grid, st, &m, a, nullptr);                          \
+                                     const StageArgs& a, bool dep) {                                    \
+    return launch_stage_tma_impl<S, C>(kind, R, ty, grid, st, &m, a, dep, nullptr);                     \
   }                                                                                                     \
   cudaError_t stage_tma_occupancy_##TAG(int kind, int R, int ty, int* ctas_per_sm) {                    \
-    return launch_stage_tma_impl<S, C>(kind, R, ty, dim3(), nullptr, nullptr, StageArgs(), ctas_per_sm); \
+    return launch_stage_tma_impl<S, C>(kind, R, ty, dim3(), nullptr, nullptr, StageArgs(), false, ctas_per_sm); \
   }                                                                                                     \
   int batch_rows_##TAG(int kind) {                                                                      \
     return (std::is_same<S, float2>::value && std::is_same<C, float>::value && is_rk4_kind(kind))          \

@@ -184,8 +184,10 @@ __host__ __device__ constexpr int single_zu() {
 }
 
 // ZU: unroll factor of the z march (the z-queue shifts are renamed across
-// ZU planes); see single_zu.
-template <class S, class C, int R, int KIND, int TY, int PY, class LY, int ZU = 1>
+// ZU planes); see single_zu.  PDL: the kernel may be launched as a dependent
+// of the previous stage (single-solve kernels; the persistent batched ones
+// have no free slots to start early in, and lost 8 % with it).
+template <class S, class C, int R, int KIND, int TY, int PY, class LY, int ZU = 1, bool PDL = false>
 __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a, int bx, int by, int bz,
                                          TmaRing& rg, int* s_abort, double& r_norm, double& r_en,
                                          double& r_err) {
@@ -240,11 +242,6 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
     __syncthreads();
   };
 
-  if (tid == 0) {
-    for (int l = 0; l < min(NSS, L); ++l) issue_stencil(l);
-    for (int m = 0; m < min(NPS, M); ++m) issue_pw(m);
-  }
-
   // per owned row: grid row, activity, centre offset in a stencil tile
   int jr[PY], cofs[PY];
   bool act[PY];
@@ -263,6 +260,12 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
   // index ranges [0, R] and [n-1-R, n-1] of an axis only.
   const bool xyg = (bx * TX <= R) || (bx * TX + TX - 1 >= g.nx - 1 - R) || (by * TY <= R) ||
                    (by * TY + TY - 1 >= g.ny - 1 - R);
+
+  if constexpr (PDL) pdl_wait();  // everything above reads host-written tables only
+  if (tid == 0) {
+    for (int l = 0; l < min(NSS, L); ++l) issue_stencil(l);
+    for (int m = 0; m < min(NPS, M); ++m) issue_pw(m);
+  }
 
   auto stile = [&](int l) { return (const S*)(rg.sring + ((SB + l) % NSS) * LY::ST_SLOT); };
   S q[PY][2 * R + 1];  // z queue of each owned row: planes k-R .. k+R
@@ -388,6 +391,7 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
     if (++pw_s == NPS) { pw_s = 0; pw_p ^= 1; }
 
     __syncthreads();  // every thread is done with stencil slot lc and point-wise slot m
+    if (PDL && m + 2 >= M) pdl_trigger();
     if (*s_abort) {
       drain(ll, m);
       return false;
@@ -412,7 +416,7 @@ __global__ void __launch_bounds__(32 * TY / PY) k_stage_tma(const __grid_constan
   __shared__ int s_abort;
   TmaRing rg = tma_ring_setup<LY>(smem_raw, &s_abort);
   double r_norm = 0.0, r_en = 0.0, r_err = 0.0;
-  if (!tma_item<S, C, R, KIND, TY, PY, LY, single_zu<S, KIND>()>(maps, a, blockIdx.x, blockIdx.y, blockIdx.z, rg,
+  if (!tma_item<S, C, R, KIND, TY, PY, LY, single_zu<S, KIND>(), true>(maps, a, blockIdx.x, blockIdx.y, blockIdx.z, rg,
                                                                   &s_abort, r_norm,
                                            r_en, r_err))
     return;
@@ -440,7 +444,7 @@ __device__ __forceinline__ void st_pair(float2* p, float2 v0, float2 v1, bool ac
     *p = v0;
 }
 
-template <class C, int R, int KIND, int TY, int PY, class LY, int ZU = 1>
+template <class C, int R, int KIND, int TY, int PY, class LY, int ZU = 1, bool PDL = false>
 __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageArgs& a, int bx, int by, int bz,
                                               TmaRing& rg, int* s_abort, double& r_norm, double& r_en,
                                               double& r_err) {
@@ -495,11 +499,6 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
     __syncthreads();
   };
 
-  if (tid == 0) {
-    for (int l = 0; l < min(NSS, L); ++l) issue_stencil(l);
-    for (int m = 0; m < min(NPS, M); ++m) issue_pw(m);
-  }
-
   int jr[PY], cofs[PY], pofs[PY], jq[NS];
   bool act[NS];
   long long o[PY], oq[NS];
@@ -522,6 +521,12 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
   }
   const bool xyg = (bx * TX <= R) || (bx * TX + TX - 1 >= g.nx - 1 - R) || (by * TY <= R) ||
                    (by * TY + TY - 1 >= g.ny - 1 - R);
+
+  if constexpr (PDL) pdl_wait();  // everything above reads host-written tables only
+  if (tid == 0) {
+    for (int l = 0; l < min(NSS, L); ++l) issue_stencil(l);
+    for (int m = 0; m < min(NPS, M); ++m) issue_pw(m);
+  }
 
   auto stile = [&](int l) { return (const S*)(rg.sring + ((SB + l) % NSS) * LY::ST_SLOT); };
   float4 q[PY][2 * R + 1];  // z queue of each owned row's pair: planes k-R .. k+R
@@ -676,6 +681,7 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
     if (++pw_s == NPS) { pw_s = 0; pw_p ^= 1; }
 
     __syncthreads();
+    if (PDL && m + 2 >= M) pdl_trigger();
     if (*s_abort) {
       drain(ll, m);
       return false;
@@ -701,7 +707,7 @@ __global__ void __launch_bounds__(16 * TY / PY) k_stage_tma_pair(const __grid_co
   __shared__ int s_abort;
   TmaRing rg = tma_ring_setup<LY>(smem_raw, &s_abort);
   double r_norm = 0.0, r_en = 0.0, r_err = 0.0;
-  if (!tma_item_pair<C, R, KIND, TY, PY, LY, single_zu<float2, KIND>()>(maps, a, blockIdx.x, blockIdx.y, blockIdx.z,
+  if (!tma_item_pair<C, R, KIND, TY, PY, LY, single_zu<float2, KIND>(), true>(maps, a, blockIdx.x, blockIdx.y, blockIdx.z,
                                                                        rg, &s_abort, r_norm,
                                              r_en, r_err))
     return;

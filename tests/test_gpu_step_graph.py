@@ -1,0 +1,36 @@
+"""A call of many fixed steps replays captured graphs of eight steps and of
+one, whose stage kernels are launched as dependents of each other; states and
+clock equal those of one call per step, bitwise, for every remainder."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from gpe_b200.solver import RunParams, Solver
+
+pytestmark = pytest.mark.gpu
+
+
+# (20, 18, 16) one thread per site; (72, 70, 66) the march, several CTAs per SM
+@pytest.mark.parametrize("shape", [(20, 18, 16), (72, 70, 66)])
+@pytest.mark.parametrize("storage,scheme", [("c128", "rk4"), ("c64", "rk4"), ("c128", "rk2")])
+def test_many_steps_equal_single_calls(gpu, shape, storage, scheme):
+    nx, ny, nz = shape
+    rp = RunParams(nx=nx, ny=ny, nz=nz, xr=0.25 * (nx - 1), yr=0.25 * (ny - 1), zr=0.25 * (nz - 1), tau=0.004,
+                   scheme=scheme, eqn_to_solve=2, bcs=1, order=4, Urhs=0.1, storage=storage)
+    rng = np.random.default_rng(nx)
+    psi0 = 1.0 + 0.1 * (rng.normal(size=(nz, ny, nx)) + 1j * rng.normal(size=(nz, ny, nx)))
+    one, many = Solver(rp), Solver(rp)
+    one.set_state(psi0)
+    many.set_state(psi0)
+    for n in (2, 3, 8, 9, 10, 11, 17, 18, 25):
+        for _ in range(n - 1):
+            one.solver(1)
+        a = one.solver(1, want_norm=n % 2 == 0)
+        b = many.solver(n, want_norm=n % 2 == 0)
+        np.testing.assert_array_equal(many.get_state(), one.get_state(), err_msg=f"{n} steps")
+        assert (one.t, one.p) == (many.t, many.p) and b.accepted == n
+        if n % 2 == 0:
+            assert a.norm == b.norm
+    one.close()
+    many.close()
