@@ -103,8 +103,8 @@ Shells shells() {
 // neighbours: a segmented scan sums them and the last lane of each segment
 // adds to the warp's histogram.  Shell sums and counts stay in registers.
 // tot uses the reference's real-space-indexed k grid (kq tables), one term
-// per mode.  256^3: 1004 us with a 32-step lane loop per mode and bin,
-// (one read of 256 MiB takes 41; the FP64 divisions of tot bound it).
+// per mode.  256^3: 1004 us with a 32-step lane loop per mode and bin, 112 us
+// so (one read of 256 MiB takes 41; the FP64 divisions of tot bound it).
 __global__ void __launch_bounds__(FFT_THREADS) k_spectrum(const double2* __restrict__ raw, int nx, int ny, int nz,
                                                           const double* __restrict__ kq, int nbins,
                                                           int want_spectrum, Shells th, double* part) {
