@@ -33,28 +33,25 @@ __device__ __forceinline__ double rr_of(double r) {
   return sqrt((0.3437 + 0.0286 * r2) / ((1.0 + 0.3333 * r2) + 0.0286 * r4));
 }
 
-// get_r / get_theta (src/ic.f90:735-889) for a line along dir
+// get_r / get_theta (src/ic.f90:735-889) for a line along dir: the scaled
+// distance r from the line and e^{i theta}, theta = sgn atan2(sc b, sc a).  An
+// unperturbed line evaluates no sine of its displacement.
 __device__ __forceinline__ void line_geom(const gpe_line& vl, double sc, double x, double y, double z, double* r,
-                                          double* th) {
+                                          double* cth, double* sth) {
   const double eps = 2.220446049250313e-16;
   double s1 = 0.0, s2 = 0.0;
   if (fabs(vl.ll) < eps) {
     s1 = 1.0;
     s2 = 1.0;
   }
-  double a, b;
-  if (vl.dir == 'x') {
-    a = y - vl.y0 - vl.amp1 * sin(2.0 * kPi * (x - vl.x0) / (vl.ll + s1));
-    b = z - vl.z0 - vl.amp2 * cos(2.0 * kPi * (x - vl.x0) / (vl.ll + s2));
-  } else if (vl.dir == 'y') {
-    a = z - vl.z0 - vl.amp1 * sin(2.0 * kPi * (y - vl.y0) / (vl.ll + s1));
-    b = x - vl.x0 - vl.amp2 * cos(2.0 * kPi * (y - vl.y0) / (vl.ll + s2));
-  } else {
-    a = x - vl.x0 - vl.amp1 * sin(2.0 * kPi * (z - vl.z0) / (vl.ll + s1));
-    b = y - vl.y0 - vl.amp2 * cos(2.0 * kPi * (z - vl.z0) / (vl.ll + s2));
-  }
+  double a, b, along;
+  if (vl.dir == 'x') { a = y - vl.y0; b = z - vl.z0; along = x - vl.x0; }
+  else if (vl.dir == 'y') { a = z - vl.z0; b = x - vl.x0; along = y - vl.y0; }
+  else { a = x - vl.x0; b = y - vl.y0; along = z - vl.z0; }
+  if (vl.amp1 != 0.0) a -= vl.amp1 * sin(2.0 * kPi * along / (vl.ll + s1));
+  if (vl.amp2 != 0.0) b -= vl.amp2 * cos(2.0 * kPi * along / (vl.ll + s2));
   *r = sqrt(sc * (a * a) + sc * (b * b));
-  *th = vl.sgn * atan2(sc * b, sc * a);
+  sincos(vl.sgn * atan2(sc * b, sc * a), sth, cth);
 }
 
 // vortex_ring (src/ic.f90:357-514)
@@ -64,10 +61,13 @@ __device__ __forceinline__ void ring_val(const gpe_ring& vr, double sc, double x
   if (vr.plane[0] == 'x' && vr.plane[1] == 'y') { u = x; v = y; w = z; u0 = vr.x0; v0 = vr.y0; w0 = vr.z0; }
   else if (vr.plane[0] == 'x' && vr.plane[1] == 'z') { u = x; v = z; w = y; u0 = vr.x0; v0 = vr.z0; w0 = vr.y0; }
   else { u = y; v = z; w = x; u0 = vr.y0; v0 = vr.z0; w0 = vr.x0; }
-  const double theta = atan2(v - v0, u - u0);
-  const double s = sqrt((u - u0) * (u - u0) + (v - v0) * (v - v0)) - vr.r1 * sin((double)vr.kk * theta);
-  const double dist = vr.amp * cos((double)vr.mm * theta);
-  const double pp = w - vr.r1 * cos((double)vr.kk * theta);
+  double s = sqrt((u - u0) * (u - u0) + (v - v0) * (v - v0)), dist = 0.0, pp = w;
+  if (vr.r1 != 0.0 || vr.amp != 0.0) {  // a perturbed ring: the angle enters
+    const double theta = atan2(v - v0, u - u0);
+    s -= vr.r1 * sin((double)vr.kk * theta);
+    dist = vr.amp * cos((double)vr.mm * theta);
+    pp -= vr.r1 * cos((double)vr.kk * theta);
+  }
   const double A = sc * (pp - w0), Bp = sc * ((s + vr.r0) - dist), Bm = sc * ((s - vr.r0) - dist);
   const double q1 = rr_of(sqrt(A * A + Bp * Bp)), q2 = rr_of(sqrt(A * A + Bm * Bm));
   const double z1r = A + vr.dir * 0.0 * Bp, z1i = vr.dir * Bp;
@@ -114,83 +114,181 @@ __device__ __forceinline__ void pair_val(double x, double y, double* re, double*
   *im = (x * ((b0 + b1 * x2) + b2 * y2)) / denom;
 }
 
-// The product of the closed-form factors of ic at (x, y, z), factors taken
-// left to right as the reference's init_cond expression multiplies them.
-__device__ __forceinline__ void ic_product(const gpe_ic& ic, const IcGrid& G, double x, double y, double z,
-                                           double* out_r, double* out_i) {
-    double pr = 1.0, pi = 0.0;
-    for (int q = 0; q < ic.nfactors; ++q) {
-      double fr = 1.0, fi = 0.0;
-      switch (ic.factor[q]) {
-        case GPE_IC_FERMI: {
-          const double v = 0.5 * (((G.omx * G.omx) * (x * x) + (G.omy * G.omy) * (y * y)) + (G.omz * G.omz) * (z * z));
-          const double a = (G.mu - v) / G.g;
-          fr = a >= 0.0 ? sqrt(a) : 0.0;
-          break;
-        }
-        case GPE_IC_LINE: {
-          double r, th;
-          line_geom(ic.line, G.scal, x, y, z, &r, &th);
-          const double a = ic.line.imprint_phase ? 1.0 : 1.0 - exp(-0.7 * pow(r, 1.15));
-          fr = a * cos(th);
-          fi = a * sin(th);
-          break;
-        }
-        case GPE_IC_LINE_PADE: {
-          double r, th;
-          line_geom(ic.line, G.scal, x, y, z, &r, &th);
-          const double a = r * rr_of(r);
-          fr = a * cos(th);
-          fi = a * sin(th);
-          break;
-        }
-        case GPE_IC_RING:
-          ring_val(ic.ring, G.scal, x, y, z, &fr, &fi);
-          break;
-        case GPE_IC_PADE_PULSE:
-        case GPE_IC_PADE_RING:
-          pade_val(ic.factor[q] == GPE_IC_PADE_PULSE, ic.pulse, x, y, z, &fr, &fi);
-          break;
-        case GPE_IC_VORTEX_PAIR:
-          pair_val(x, y, &fr, &fi);
-          break;
-        case GPE_IC_SPHERE:  // ic.f90:640-662 (rad = 10, eps1 = 2)
-          fr = 0.5 * (1.0 + tanh((sqrt((x * x + y * y) + z * z) - 10.0) - 2.0));
-          break;
-        case GPE_IC_SPHERE2:  // ic.f90:666-684 (amp = 100, width = 10)
-          fr = 100.0 * exp(-((x * x + y * y) + z * z) / 10.0);
-          break;
-        case GPE_IC_WALL:  // ic.f90:688-709 (pos = -30)
-          fr = z <= -30.0 ? 0.0 : 1.0;
-          break;
-        default:
-          break;
+// fermi (src/ic.f90:278): sqrt(max(mu - V, 0)/g) with vxy = omx^2 x^2 + omy^2 y^2
+__device__ __forceinline__ double fermi_val(const IcGrid& G, double vxy, double z) {
+  const double v = 0.5 * (vxy + (G.omz * G.omz) * (z * z));
+  const double a = (G.mu - v) / G.g;
+  return a >= 0.0 ? sqrt(a) : 0.0;
+}
+
+// Closed-form factor q of ic at (x, y, z).
+__device__ __forceinline__ void ic_factor(const gpe_ic& ic, int q, const IcGrid& G, double x, double y, double z,
+                                          double* out_r, double* out_i) {
+  double fr = 1.0, fi = 0.0;
+  switch (ic.factor[q]) {
+    case GPE_IC_FERMI:
+      fr = fermi_val(G, (G.omx * G.omx) * (x * x) + (G.omy * G.omy) * (y * y), z);
+      break;
+    case GPE_IC_LINE: {
+      double r, c, s;
+      line_geom(ic.line, G.scal, x, y, z, &r, &c, &s);
+      const double a = ic.line.imprint_phase ? 1.0 : 1.0 - exp(-0.7 * pow(r, 1.15));
+      fr = a * c;
+      fi = a * s;
+      break;
+    }
+    case GPE_IC_LINE_PADE: {
+      double r, c, s;
+      line_geom(ic.line, G.scal, x, y, z, &r, &c, &s);
+      const double a = r * rr_of(r);
+      fr = a * c;
+      fi = a * s;
+      break;
+    }
+    case GPE_IC_RING:
+      ring_val(ic.ring, G.scal, x, y, z, &fr, &fi);
+      break;
+    case GPE_IC_PADE_PULSE:
+    case GPE_IC_PADE_RING:
+      pade_val(ic.factor[q] == GPE_IC_PADE_PULSE, ic.pulse, x, y, z, &fr, &fi);
+      break;
+    case GPE_IC_VORTEX_PAIR:
+      pair_val(x, y, &fr, &fi);
+      break;
+    case GPE_IC_SPHERE:  // ic.f90:640-662 (rad = 10, eps1 = 2)
+      fr = 0.5 * (1.0 + tanh((sqrt((x * x + y * y) + z * z) - 10.0) - 2.0));
+      break;
+    case GPE_IC_SPHERE2:  // ic.f90:666-684 (amp = 100, width = 10)
+      fr = 100.0 * exp(-((x * x + y * y) + z * z) / 10.0);
+      break;
+    case GPE_IC_WALL:  // ic.f90:688-709 (pos = -30)
+      fr = z <= -30.0 ? 0.0 : 1.0;
+      break;
+    default:
+      break;
+  }
+  *out_r = fr;
+  *out_i = fi;
+}
+
+// Is factor q the same on every plane of a column?
+__device__ __forceinline__ bool ic_columnar(const gpe_ic& ic, int q) {
+  const int f = ic.factor[q];
+  if (f == GPE_IC_UNIFORM || f == GPE_IC_VORTEX_PAIR) return true;
+  return (f == GPE_IC_LINE || f == GPE_IC_LINE_PADE) && ic.line.dir == 'z' && ic.line.amp1 == 0.0 && ic.line.amp2 == 0.0;
+}
+
+constexpr int IC_TY = 8;       // rows of a block of 32 x IC_TY columns
+constexpr int IC_CTAS = 3;     // blocks per SM the registers are fitted to
+constexpr int IC_PLANES = 16;  // most planes a thread takes of its column
+constexpr int IC_MAX = 4;      // factors of a product
+
+// Planes per thread: as many as leave the device IC_CTAS blocks per SM, at
+// most IC_PLANES (beyond that the column's factors cost little anyway).
+int ic_planes(const Geom& g) {
+  const long long tiles = (long long)((g.nx + 31) / 32) * ((g.ny + IC_TY - 1) / IC_TY);
+  const long long chunks = (148LL * IC_CTAS + tiles - 1) / tiles;
+  const int z = (int)(g.nz / chunks);
+  return z < 1 ? 1 : (z > IC_PLANES ? IC_PLANES : z);
+}
+
+dim3 ic_blocks(const Geom& g) {
+  const int z = ic_planes(g);
+  return dim3((g.nx + 31) / 32, (g.ny + IC_TY - 1) / IC_TY, (g.nz + z - 1) / z);
+}
+
+// The product of the closed-form factors, taken left to right as the
+// reference's init_cond expression multiplies them, over `planes` planes of
+// one column (MULT: times the state there, or its modulus).  A thread keeps
+// the factors that do not depend on z, so a vortex line along z costs its core
+// and phase once per column; products of those and fermi run in a loop of
+// their own without the other factors' code, and there is no index division.
+// Instruction issue bounds it.  set_ic on 192 x 192 x 384 complex128, us, with
+// every factor (and an arc tangent, a sine and a cosine) per site / so:
+// fermi x line_pade 958 / 72, fermi x line 1104 / 79, ring 1027 / 298.
+template <class S, bool MULT>
+__device__ __forceinline__ void ic_column(S* f, const Geom& g, int R, int bcs, const IcGrid& G, const gpe_ic& ic,
+                                          int planes, int modulus) {
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * IC_TY + threadIdx.y;
+  if (i >= g.nx || j >= g.ny) return;
+  const int k0 = blockIdx.z * planes, k1 = min(k0 + planes, g.nz);
+  const double x = coord(G.xl, G.dx, i), y = coord(G.yl, G.dy, j);
+  const double vxy = (G.omx * G.omx) * (x * x) + (G.omy * G.omy) * (y * y);
+  double fr[IC_MAX], fi[IC_MAX];
+  bool other = false;  // a factor that changes along the column and is not fermi
+#pragma unroll
+  for (int q = 0; q < IC_MAX; ++q) {
+    fr[q] = 1.0;
+    fi[q] = 0.0;
+    if (q >= ic.nfactors) continue;
+    if (ic_columnar(ic, q)) ic_factor(ic, q, G, x, y, 0.0, &fr[q], &fi[q]);
+    else other |= ic.factor[q] != GPE_IC_FERMI;
+  }
+
+  const int gx = ghost_pos(i, g.nx, R, bcs), gy = ghost_pos(j, g.ny, R, bcs);
+  S* p = f + (long long)(k0 + 2) * g.pz + (long long)(j + 2) * g.px + g.xoff + i;
+  const long long ox = gx - i, oy = (long long)(gy - j) * g.px;
+  auto put = [&](int k, double pr, double pi) {
+    if constexpr (MULT) {
+      double ar = (double)p->x, ai = (double)p->y;
+      if (modulus) {
+        ar = hypot(ar, ai);
+        ai = 0.0;
       }
-      const double nr = pr * fr - pi * fi, ni = pr * fi + pi * fr;
+      const double nr = ar * pr - ai * pi, ni = ar * pi + ai * pr;
       pr = nr;
       pi = ni;
     }
-    *out_r = pr;
-    *out_i = pi;
-}
-
-template <class S>
-__global__ void k_ic_closed_form(S* f, Geom g, int R, int bcs, IcGrid G, gpe_ic ic) {
-  const long long n = (long long)g.nx * g.ny * g.nz;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % g.nx);
-    const long long rq = t / g.nx;
-    const int j = (int)(rq % g.ny);
-    const int k = (int)(rq / g.ny);
-    const double x = coord(G.xl, G.dx, i), y = coord(G.yl, G.dy, j), z = coord(G.zl, G.dz, k);
-    double pr, pi;
-    ic_product(ic, G, x, y, z, &pr, &pi);
     S s;
     s.x = (typename Stor<S>::R)pr;
     s.y = (typename Stor<S>::R)pi;
-    store_with_ghosts(f, g, (long long)(j + 2) * g.px + g.xoff + i, i, j, k, ghost_pos(i, g.nx, R, bcs),
-                      ghost_pos(j, g.ny, R, bcs), ghost_pos(k, g.nz, R, bcs), s);
+    *p = s;
+    if (gx != NOGHOST) p[ox] = s;
+    if (gy != NOGHOST) p[oy] = s;
+    if (k <= R || k >= g.nz - 1 - R) {
+      const int gz = ghost_pos(k, g.nz, R, bcs);
+      if (gz != NOGHOST) p[(long long)(gz - k) * g.pz] = s;
+    }
+    p += g.pz;
+  };
+  if (!other) {
+#pragma unroll 2
+    for (int k = k0; k < k1; ++k) {
+      const double fv = fermi_val(G, vxy, coord(G.zl, G.dz, k));
+      double pr = 1.0, pi = 0.0;
+#pragma unroll
+      for (int q = 0; q < IC_MAX; ++q) {
+        if (q >= ic.nfactors) break;
+        const double ar = ic.factor[q] == GPE_IC_FERMI ? fv : fr[q], ai = fi[q];
+        const double nr = pr * ar - pi * ai, ni = pr * ai + pi * ar;
+        pr = nr;
+        pi = ni;
+      }
+      put(k, pr, pi);
+    }
+  } else {
+    for (int k = k0; k < k1; ++k) {
+      const double z = coord(G.zl, G.dz, k);
+      double pr = 1.0, pi = 0.0;
+#pragma unroll
+      for (int q = 0; q < IC_MAX; ++q) {
+        if (q >= ic.nfactors) break;
+        double ar = fr[q], ai = fi[q];
+        if (!ic_columnar(ic, q)) ic_factor(ic, q, G, x, y, z, &ar, &ai);
+        const double nr = pr * ar - pi * ai, ni = pr * ai + pi * ar;
+        pr = nr;
+        pi = ni;
+      }
+      put(k, pr, pi);
+    }
   }
+}
+
+template <class S>
+__global__ void __launch_bounds__(32 * IC_TY, IC_CTAS) k_ic_closed_form(S* f, Geom g, int R, int bcs, IcGrid G,
+                                                                        const __grid_constant__ gpe_ic ic,
+                                                                        int planes) {
+  ic_column<S, false>(f, g, R, bcs, G, ic, planes, 0);
 }
 
 // psi <- psi * IC (modulus = 0: the state_restart product with init_cond,
@@ -198,29 +296,10 @@ __global__ void k_ic_closed_form(S* f, Geom g, int R, int bcs, IcGrid G, gpe_ic 
 // imprint_vortex_line, src/variables.f90:1166-1180), in FP64 per site, the
 // new value stored with its ghosts.
 template <class S>
-__global__ void k_ic_multiply(S* f, Geom g, int R, int bcs, IcGrid G, gpe_ic ic, int modulus) {
-  const long long n = (long long)g.nx * g.ny * g.nz;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % g.nx);
-    const long long rq = t / g.nx;
-    const int j = (int)(rq % g.ny);
-    const int k = (int)(rq / g.ny);
-    const double x = coord(G.xl, G.dx, i), y = coord(G.yl, G.dy, j), z = coord(G.zl, G.dz, k);
-    double pr, pi;
-    ic_product(ic, G, x, y, z, &pr, &pi);
-    const long long col = (long long)(j + 2) * g.px + g.xoff + i;
-    const S v = f[(long long)(k + 2) * g.pz + col];
-    double ar = (double)v.x, ai = (double)v.y;
-    if (modulus) {
-      ar = hypot(ar, ai);
-      ai = 0.0;
-    }
-    S s;
-    s.x = (typename Stor<S>::R)(ar * pr - ai * pi);
-    s.y = (typename Stor<S>::R)(ar * pi + ai * pr);
-    store_with_ghosts(f, g, col, i, j, k, ghost_pos(i, g.nx, R, bcs), ghost_pos(j, g.ny, R, bcs),
-                      ghost_pos(k, g.nz, R, bcs), s);
-  }
+__global__ void __launch_bounds__(32 * IC_TY, IC_CTAS) k_ic_multiply(S* f, Geom g, int R, int bcs, IcGrid G,
+                                                                     const __grid_constant__ gpe_ic ic, int planes,
+                                                                     int modulus) {
+  ic_column<S, true>(f, g, R, bcs, G, ic, planes, modulus);
 }
 
 __device__ __forceinline__ unsigned long long splitmix64(unsigned long long seed, unsigned long long idx) {
@@ -387,9 +466,9 @@ cudaError_t ic_multiply(const gpe_params& p, const Geom& g, int esz, int R, cons
                         int modulus, cudaStream_t st) {
   if (ic_needs_fft(&ic)) return cudaErrorInvalidValue;
   const IcGrid G = ic_grid(p);
-  const int nb = 148 * 8;
-  if (esz == 16) k_ic_multiply<double2><<<nb, 256, 0, st>>>((double2*)psi_field, g, R, p.bcs, G, ic, modulus);
-  else k_ic_multiply<float2><<<nb, 256, 0, st>>>((float2*)psi_field, g, R, p.bcs, G, ic, modulus);
+  const dim3 nb = ic_blocks(g), nt(32, IC_TY);
+  if (esz == 16) k_ic_multiply<double2><<<nb, nt, 0, st>>>((double2*)psi_field, g, R, p.bcs, G, ic, ic_planes(g), modulus);
+  else k_ic_multiply<float2><<<nb, nt, 0, st>>>((float2*)psi_field, g, R, p.bcs, G, ic, ic_planes(g), modulus);
   return cudaGetLastError();
 }
 
@@ -398,8 +477,9 @@ cudaError_t ic_generate(const gpe_params& p, const Geom& g, int esz, int R, cons
   const IcGrid G = ic_grid(p);
   const int nb = 148 * 8;
   if (!ic_needs_fft(&ic)) {
-    if (esz == 16) k_ic_closed_form<double2><<<nb, 256, 0, st>>>((double2*)psi_field, g, R, p.bcs, G, ic);
-    else k_ic_closed_form<float2><<<nb, 256, 0, st>>>((float2*)psi_field, g, R, p.bcs, G, ic);
+    const dim3 cb = ic_blocks(g), nt(32, IC_TY);
+    if (esz == 16) k_ic_closed_form<double2><<<cb, nt, 0, st>>>((double2*)psi_field, g, R, p.bcs, G, ic, ic_planes(g));
+    else k_ic_closed_form<float2><<<cb, nt, 0, st>>>((float2*)psi_field, g, R, p.bcs, G, ic, ic_planes(g));
     return cudaGetLastError();
   }
   const long long n = (long long)p.nx * p.ny * p.nz;
