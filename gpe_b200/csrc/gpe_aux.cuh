@@ -6,41 +6,85 @@
 
 namespace gpe {
 
-// contiguous interior (complex T2, [k][j][i]) -> ghost-padded field S with
-// its face ghosts (the halo exchange of gpe.f90:173-176, done once)
-template <class S, class T2>
-__global__ void k_pack(const T2* __restrict__ src, S* __restrict__ dst, Geom g, int R, int bcs, int zmask = 3) {
-  const long long n = (long long)g.nx * g.ny * g.nz;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % g.nx);
-    const long long r = t / g.nx;
-    const int j = (int)(r % g.ny);
-    const int k = (int)(r / g.ny);
-    const T2 v = src[t];
-    S s;
-    s.x = (typename Stor<S>::R)v.x;
-    s.y = (typename Stor<S>::R)v.y;
-    const long long col = (long long)(j + 2) * g.px + g.xoff + i;
-    store_with_ghosts(dst, g, col, i, j, k, ghost_pos(i, g.nx, R, bcs), ghost_pos(j, g.ny, R, bcs),
-                      zghost_pos(k, g.nz, R, bcs, zmask), s);
+// Launch shape of the row kernels below: a warp takes a row at a time, lanes
+// along x.  Index arithmetic is per row, not a 64-bit division per site, and a
+// lane has several independent loads in flight.
+constexpr int ROW_THREADS = 256;
+constexpr int ROW_GRID = 148 * 8;
+
+// f(row k, row j, lane): every interior row once, a warp each
+template <class F>
+__device__ __forceinline__ void for_each_row(const Geom& g, F f) {
+  const int lane = threadIdx.x & 31;
+  const long long rows = (long long)g.ny * g.nz;
+  const int tw = gridDim.x * (ROW_THREADS / 32);
+  for (long long r = blockIdx.x * (ROW_THREADS / 32) + (threadIdx.x >> 5); r < rows; r += tw) {
+    const int k = (int)(r / g.ny), j = (int)(r - (long long)k * g.ny);
+    f(k, j, lane, r);
   }
+}
+
+// Store a row's values (val(i) for lanes of x) with their face ghosts: whole
+// images of the row in y and z, the first and last sites in x.
+template <class S, class F>
+__device__ __forceinline__ void put_row(S* __restrict__ f, const Geom& g, int R, int bcs, int zmask, int k, int j,
+                                        int lane, F val) {
+  S* row = f + (long long)(k + 2) * g.pz + (long long)(j + 2) * g.px + g.xoff;
+  const int gy = ghost_pos(j, g.ny, R, bcs), gz = zghost_pos(k, g.nz, R, bcs, zmask);
+  S* yrow = gy == NOGHOST ? nullptr : row + (long long)(gy - j) * g.px;
+  S* zrow = gz == NOGHOST ? nullptr : row + (long long)(gz - k) * g.pz;
+  for (int i0 = lane; i0 < g.nx; i0 += 4 * 32) {
+    S s[4];  // the loads of four chunks before any store
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (i0 + 32 * c < g.nx) s[c] = val(i0 + 32 * c);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int i = i0 + 32 * c;
+      if (i >= g.nx) break;
+      row[i] = s[c];
+      if (yrow) yrow[i] = s[c];
+      if (zrow) zrow[i] = s[c];
+      const int gx = ghost_pos(i, g.nx, R, bcs);
+      if (gx != NOGHOST) row[gx] = s[c];
+    }
+  }
+}
+
+// contiguous interior (complex T2, [k][j][i]) -> ghost-padded field S with
+// its face ghosts (the halo exchange of gpe.f90:173-176, done once).  256^3
+// complex128: 124 us with an index division per site, 84 us so (82 at the copy
+// rate).
+template <class S, class T2>
+__global__ void __launch_bounds__(ROW_THREADS) k_pack(const T2* __restrict__ src, S* __restrict__ dst, Geom g, int R,
+                                                      int bcs, int zmask = 3) {
+  for_each_row(g, [&](int k, int j, int lane, long long r) {
+    const T2* p = src + r * g.nx;
+    put_row(dst, g, R, bcs, zmask, k, j, lane, [&](int i) {
+      const T2 v = p[i];
+      S s;
+      s.x = (typename Stor<S>::R)v.x;
+      s.y = (typename Stor<S>::R)v.y;
+      return s;
+    });
+  });
 }
 
 // ghost-padded field -> contiguous interior
 template <class S, class T2>
-__global__ void k_unpack(const S* __restrict__ src, T2* __restrict__ dst, Geom g) {
-  const long long n = (long long)g.nx * g.ny * g.nz;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % g.nx);
-    const long long r = t / g.nx;
-    const int j = (int)(r % g.ny);
-    const int k = (int)(r / g.ny);
-    const S v = src[(long long)(k + 2) * g.pz + (long long)(j + 2) * g.px + g.xoff + i];
-    T2 o;
-    o.x = v.x;
-    o.y = v.y;
-    dst[t] = o;
-  }
+__global__ void __launch_bounds__(ROW_THREADS) k_unpack(const S* __restrict__ src, T2* __restrict__ dst, Geom g) {
+  for_each_row(g, [&](int k, int j, int lane, long long r) {
+    const S* row = src + (long long)(k + 2) * g.pz + (long long)(j + 2) * g.px + g.xoff;
+    T2* p = dst + r * g.nx;
+#pragma unroll 4
+    for (int i = lane; i < g.nx; i += 32) {
+      const S v = row[i];
+      T2 o;
+      o.x = v.x;
+      o.y = v.y;
+      p[i] = o;
+    }
+  });
 }
 
 // get_norm partials (variables.f90:554-576): w_i w_j w_k |psi|^2 per block,
@@ -126,24 +170,31 @@ static __global__ void __launch_bounds__(256) k_finalize_ranges(const double* __
 }
 
 // Face ghosts of a field whose interior was just written (for example by a
-// strided host-to-device copy): every interior site writes its ghost copies.
+// strided host-to-device copy).  Rows away from the y and z faces touch their
+// first and last R + 1 sites only.  256^3 complex128: 102 us with a scan of the
+// interior, 43 us so.
 template <class S>
-__global__ void k_fill_ghosts(S* f, Geom g, int R, int bcs) {
-  const long long n = (long long)g.nx * g.ny * g.nz;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % g.nx);
-    const long long r = t / g.nx;
-    const int j = (int)(r % g.ny);
-    const int k = (int)(r / g.ny);
-    const int gx = ghost_pos(i, g.nx, R, bcs), gy = ghost_pos(j, g.ny, R, bcs), gz = ghost_pos(k, g.nz, R, bcs);
-    if (gx == NOGHOST && gy == NOGHOST && gz == NOGHOST) continue;
-    const long long col = (long long)(j + 2) * g.px + g.xoff + i;
-    const long long pl = (long long)(k + 2) * g.pz;
-    const S v = f[pl + col];
-    if (gx != NOGHOST) f[pl + (long long)(j + 2) * g.px + g.xoff + gx] = v;
-    if (gy != NOGHOST) f[pl + (long long)(gy + 2) * g.px + g.xoff + i] = v;
-    if (gz != NOGHOST) f[(long long)(gz + 2) * g.pz + col] = v;
-  }
+__global__ void __launch_bounds__(ROW_THREADS) k_fill_ghosts(S* f, Geom g, int R, int bcs) {
+  for_each_row(g, [&](int k, int j, int lane, long long) {
+    S* row = f + (long long)(k + 2) * g.pz + (long long)(j + 2) * g.px + g.xoff;
+    const int gy = ghost_pos(j, g.ny, R, bcs), gz = ghost_pos(k, g.nz, R, bcs);
+    if (gy == NOGHOST && gz == NOGHOST) {
+      // sites 0 .. R and nx-1-R .. nx-1 (nx >= 6 keeps the two ends apart)
+      const int i = lane <= R ? lane : g.nx - 2 - 2 * R + lane;
+      if (lane < 2 * R + 2 && i < g.nx) {
+        const int gx = ghost_pos(i, g.nx, R, bcs);
+        if (gx != NOGHOST) row[gx] = row[i];
+      }
+      return;
+    }
+    for (int i = lane; i < g.nx; i += 32) {
+      const S v = row[i];
+      const int gx = ghost_pos(i, g.nx, R, bcs);
+      if (gx != NOGHOST) row[gx] = v;
+      if (gy != NOGHOST) row[(long long)(gy - j) * g.px + i] = v;
+      if (gz != NOGHOST) row[(long long)(gz - k) * g.pz + i] = v;
+    }
+  });
 }
 
 // renormalise (variables.f90:715-726): var = sqrt(nn)*var/sqrt(norm), over

@@ -11,6 +11,7 @@
 #include <mutex>
 #include <tuple>
 
+#include "gpe_aux.cuh"
 #include "gpe_ic.h"
 
 namespace gpe {
@@ -311,25 +312,26 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long seed
 
 // psi_hat(m) = exp(i 2 pi u_m) for |k_m| < kc, else 0; modes in numpy's
 // fftfreq order, u_m from SplitMix64 over the linear mode index
-__global__ void k_random_spectrum(double2* buf, int nx, int ny, int nz, double dx, double dy, double dz,
-                                  unsigned long long seed, double kc) {
-  const long long n = (long long)nx * ny * nz;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % nx);
-    const long long rq = t / nx;
-    const int j = (int)(rq % ny);
-    const int k = (int)(rq / ny);
-    const int mi = i < (nx + 1) / 2 ? i : i - nx, mj = j < (ny + 1) / 2 ? j : j - ny, mk = k < (nz + 1) / 2 ? k : k - nz;
-    const double kx = 2.0 * kPi * mi / (nx * dx), ky = 2.0 * kPi * mj / (ny * dy), kz = 2.0 * kPi * mk / (nz * dz);
-    const double k2 = (kz * kz + ky * ky) + kx * kx;
-    double2 v = make_double2(0.0, 0.0);
-    if (k2 < kc * kc) {
-      const double u = (double)(splitmix64(seed, (unsigned long long)t) >> 11) * (1.0 / 9007199254740992.0);
-      const double th = 2.0 * kPi * u;
-      v = make_double2(cos(th), sin(th));
+__global__ void __launch_bounds__(ROW_THREADS) k_random_spectrum(double2* buf, Geom g, double dx, double dy, double dz,
+                                                                 unsigned long long seed, double kc) {
+  const int nx = g.nx, ny = g.ny, nz = g.nz;
+  for_each_row(g, [&](int k, int j, int lane, long long r) {
+    const int mj = j < (ny + 1) / 2 ? j : j - ny, mk = k < (nz + 1) / 2 ? k : k - nz;
+    const double ky = 2.0 * kPi * mj / (ny * dy), kz = 2.0 * kPi * mk / (nz * dz);
+    const double kyz = kz * kz + ky * ky;
+    for (int i = lane; i < nx; i += 32) {
+      const int mi = i < (nx + 1) / 2 ? i : i - nx;
+      const double kx = 2.0 * kPi * mi / (nx * dx);
+      const long long t = r * nx + i;
+      double2 v = make_double2(0.0, 0.0);
+      if (kyz + kx * kx < kc * kc) {
+        const double u = (double)(splitmix64(seed, (unsigned long long)t) >> 11) * (1.0 / 9007199254740992.0);
+        const double th = 2.0 * kPi * u;
+        v = make_double2(cos(th), sin(th));
+      }
+      buf[t] = v;
     }
-    buf[t] = v;
-  }
+  });
 }
 
 // sum |psi|^2 over the buffer (fixed-order block partials, then one block)
@@ -362,21 +364,21 @@ __global__ void __launch_bounds__(256) k_sum_parts(double* part, int nb) {
 
 // psi = buf * sqrt(n / sum|buf|^2) into the padded field with ghosts
 template <class S>
-__global__ void k_pack_scaled(const double2* __restrict__ buf, const double* __restrict__ total, S* f, Geom g,
-                              int R, int bcs) {
-  const long long n = (long long)g.nx * g.ny * g.nz;
-  const double sc = 1.0 / sqrt(*total / (double)n);
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % g.nx);
-    const long long rq = t / g.nx;
-    const int j = (int)(rq % g.ny);
-    const int k = (int)(rq / g.ny);
-    S s;
-    s.x = (typename Stor<S>::R)(buf[t].x * sc);
-    s.y = (typename Stor<S>::R)(buf[t].y * sc);
-    store_with_ghosts(f, g, (long long)(j + 2) * g.px + g.xoff + i, i, j, k, ghost_pos(i, g.nx, R, bcs),
-                      ghost_pos(j, g.ny, R, bcs), ghost_pos(k, g.nz, R, bcs), s);
-  }
+__global__ void __launch_bounds__(ROW_THREADS) k_pack_scaled(const double2* __restrict__ buf,
+                                                             const double* __restrict__ total, S* f, Geom g, int R,
+                                                             int bcs) {
+  const double n = (double)g.nx * (double)g.ny * (double)g.nz;
+  const double sc = 1.0 / sqrt(*total / n);
+  for_each_row(g, [&](int k, int j, int lane, long long r) {
+    const double2* p = buf + r * g.nx;
+    put_row(f, g, R, bcs, 3, k, j, lane, [&](int i) {
+      const double2 v = p[i];
+      S s;
+      s.x = (typename Stor<S>::R)(v.x * sc);
+      s.y = (typename Stor<S>::R)(v.y * sc);
+      return s;
+    });
+  });
 }
 
 // 3-D Z2Z plans, one per (device, grid), created on first use
@@ -475,7 +477,7 @@ cudaError_t ic_multiply(const gpe_params& p, const Geom& g, int esz, int R, cons
 cudaError_t ic_generate(const gpe_params& p, const Geom& g, int esz, int R, const gpe_ic& ic, void* psi_field,
                         void* work, size_t work_bytes, cudaStream_t st) {
   const IcGrid G = ic_grid(p);
-  const int nb = 148 * 8;
+  const int nb = ROW_GRID;
   if (!ic_needs_fft(&ic)) {
     const dim3 cb = ic_blocks(g), nt(32, IC_TY);
     if (esz == 16) k_ic_closed_form<double2><<<cb, nt, 0, st>>>((double2*)psi_field, g, R, p.bcs, G, ic, ic_planes(g));
@@ -487,7 +489,7 @@ cudaError_t ic_generate(const gpe_params& p, const Geom& g, int esz, int R, cons
   if (!work || work_bytes < need) return cudaErrorInvalidValue;
   double2* buf = (double2*)work;
   double* part = (double*)((char*)work + (((size_t)n * sizeof(double2) + 255) & ~size_t(255)));
-  k_random_spectrum<<<nb, 256, 0, st>>>(buf, p.nx, p.ny, p.nz, G.dx, G.dy, G.dz, (unsigned long long)ic.seed, ic.kc);
+  k_random_spectrum<<<nb, ROW_THREADS, 0, st>>>(buf, g, G.dx, G.dy, G.dz, (unsigned long long)ic.seed, ic.kc);
   cufftHandle plan;
   if (!plan_for(p.nx, p.ny, p.nz, &plan)) return cudaErrorUnknown;
   if (cufftSetStream(plan, st) != CUFFT_SUCCESS) return cudaErrorUnknown;
@@ -496,8 +498,8 @@ cudaError_t ic_generate(const gpe_params& p, const Geom& g, int esz, int R, cons
   const int nbs = 1000;
   k_sumsq<<<nbs, 256, 0, st>>>(buf, n, part);
   k_sum_parts<<<1, 256, 0, st>>>(part, nbs);
-  if (esz == 16) k_pack_scaled<double2><<<nb, 256, 0, st>>>(buf, part + nbs, (double2*)psi_field, g, R, p.bcs);
-  else k_pack_scaled<float2><<<nb, 256, 0, st>>>(buf, part + nbs, (float2*)psi_field, g, R, p.bcs);
+  if (esz == 16) k_pack_scaled<double2><<<nb, ROW_THREADS, 0, st>>>(buf, part + nbs, (double2*)psi_field, g, R, p.bcs);
+  else k_pack_scaled<float2><<<nb, ROW_THREADS, 0, st>>>(buf, part + nbs, (float2*)psi_field, g, R, p.bcs);
   return cudaGetLastError();
 }
 

@@ -278,9 +278,9 @@ int upload_state(gpe_pool* P, Solve* s, const void* psi, int fidx) {
   m.kind = cudaMemcpyHostToDevice;
   PCU(P, cudaMemcpy3DAsync(&m, P->st));
   if (s->esz == 16)
-    k_fill_ghosts<double2><<<148 * 4, 256, 0, P->st>>>((double2*)s->f[fidx], s->g, s->R, s->p.bcs);
+    k_fill_ghosts<double2><<<ROW_GRID, ROW_THREADS, 0, P->st>>>((double2*)s->f[fidx], s->g, s->R, s->p.bcs);
   else
-    k_fill_ghosts<float2><<<148 * 4, 256, 0, P->st>>>((float2*)s->f[fidx], s->g, s->R, s->p.bcs);
+    k_fill_ghosts<float2><<<ROW_GRID, ROW_THREADS, 0, P->st>>>((float2*)s->f[fidx], s->g, s->R, s->p.bcs);
   PCU(P, cudaGetLastError());
   return GPE_OK;
 }
