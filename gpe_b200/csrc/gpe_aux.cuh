@@ -200,12 +200,20 @@ __global__ void __launch_bounds__(ROW_THREADS) k_fill_ghosts(S* f, Geom g, int R
 // renormalise (variables.f90:715-726): var = sqrt(nn)*var/sqrt(norm), over
 // the whole padded buffer (ghost copies scale identically)
 template <class S>
-__global__ void k_scale(S* f, long long n, double a, double b) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    S v = f[t];
-    v.x = (typename Stor<S>::R)(((double)v.x * a) / b);
-    v.y = (typename Stor<S>::R)(((double)v.y * a) / b);
-    f[t] = v;
+__global__ void __launch_bounds__(ROW_THREADS) k_scale(S* f, long long n, double a, double b) {
+  const long long step = (long long)gridDim.x * ROW_THREADS;
+  for (long long t = blockIdx.x * (long long)ROW_THREADS + threadIdx.x; t < n; t += 4 * step) {
+    S v[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (t + c * step < n) v[c] = f[t + c * step];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (t + c * step < n) {
+        v[c].x = (typename Stor<S>::R)(((double)v[c].x * a) / b);
+        v[c].y = (typename Stor<S>::R)(((double)v[c].y * a) / b);
+        f[t + c * step] = v[c];
+      }
   }
 }
 

@@ -68,16 +68,16 @@ struct gpe_handle {
   double* tables = nullptr;
   std::vector<double> x, y, z;
   double dx = 0, dy = 0, dz = 0;
-  double* part_a = nullptr;  // block partials (energy / first reduction)
-  double* part_b = nullptr;  // block partials (norm / errmax)
+  double* part = nullptr;    // block partials of a reduction, finalised before the next one
+  long long part_cap = 0;    // blocks it holds
   dim3 norm_grid;            // k_norm's grid: 32 x 8 tiles x z-chunks of zc planes
   long long norm_npart = 0;  // its partials
-  double* dres = nullptr;    // [6] finalised reductions
-  double* hres = nullptr;    // pinned mirror of dres
+  double* dres = nullptr;    // [6] finalised reductions, then the status word
+  double* hres = nullptr;    // pinned mirror of dres and the status word
   void* staging = nullptr;
   size_t staging_bytes = 0;
   int zc = 8;                // planes per block of k_norm
-  int zck[K_NUM] = {0};      // planes per CTA of each stage kernel the scheme uses
+  int zck[K_NUM] = {0};      // planes per CTA of each stage kernel launched so far (chunk_of)
   int nsm = 148;             // SMs of the device
   std::string err;
   // optional per-kernel timing (gpe_profile): event pairs around launches
@@ -91,7 +91,7 @@ struct gpe_handle {
   bool use_tma = true;
   int tma_ty = TILE_32x8_ROW2;  // thread layout of the TMA stage kernel (TileVariant)
   std::vector<CUtensorMap> map_halo, map_pw;  // per field
-  int* status = nullptr;                      // device status word
+  int* status = nullptr;                      // device status word (behind dres)
   // FFT diagnostics: transform scratch + the reference's k-grid symbols
   void* fft_work = nullptr;
   size_t fft_work_bytes = 0;
@@ -118,8 +118,10 @@ struct gpe_handle {
   // one captured RK4/RK2 step without reductions, replayed by gpe_step
   // (the stage arguments, dt included, are baked into the graph)
   // [0] holds one step, [1] GRAPH_STEPS of them, so that a long run pays a
-  // graph launch and its gap once per GRAPH_STEPS steps
-  cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
+  // graph launch and its gap once per GRAPH_STEPS steps; [2] one step with
+  // the norm of its result and the copy of the results to the host
+  cudaGraphExec_t step_graph[3] = {nullptr, nullptr, nullptr};
+  int64_t norm_steps = 0;  // steps with a norm so far (the second one captures)
   double graph_dr = 0, graph_di = 0;
   bool capturing = false;  // stage launches become dependents of each other
   // asynchronous state copies (gpe_set_state_async / gpe_get_state_async):
@@ -175,54 +177,64 @@ int field_of(const gpe_handle* h, const void* p) {
   return -1;
 }
 
+// Planes per CTA of a stage kernel, chosen at its first launch by the kernel's
+// CTAs per SM (the Cash-Karp stages with many point-wise inputs hold half as
+// many as the others).
+int chunk_of(gpe_handle* h, int kind) {
+  int& zc = h->zck[kind];
+  if (zc) return zc;
+  const int th = tile_rows(h->tma_ty);
+  const long long tiles = (long long)((h->p.nx + 31) / 32) * ((h->p.ny + th - 1) / th);
+  int per = 0;
+  if (h->p.tile_zc > 0) {
+    zc = std::min(h->p.tile_zc, h->p.nz);
+  } else if (h->tma_ty == TILE_SITE) {
+    zc = 1;
+  } else if (!h->use_tma) {
+    zc = default_zc(h->g, th, h->esz);
+  } else {
+    const cudaError_t e = h->cmode == CM_F64   ? stage_tma_occupancy_f64(kind, h->R, h->tma_ty, &per)
+                          : h->cmode == CM_F32 ? stage_tma_occupancy_f32(kind, h->R, h->tma_ty, &per)
+                                               : stage_tma_occupancy_f32x(kind, h->R, h->tma_ty, &per);
+    // (a kernel that cannot be queried cannot be launched either)
+    zc = balanced_zc(h->g, h->esz, h->R, tiles, (long long)h->nsm * (e == cudaSuccess && per > 0 ? per : 1));
+  }
+  return zc;
+}
+
 // grid of a stage launch: x-y tiles times z-chunks of the kind's length
-dim3 stage_grid(const gpe_handle* h, int kind) {
-  const int th = tile_rows(h->tma_ty), zc = h->zck[kind];
+dim3 stage_grid(gpe_handle* h, int kind) {
+  const int th = tile_rows(h->tma_ty), zc = chunk_of(h, kind);
   return dim3((h->p.nx + 31) / 32, (h->p.ny + th - 1) / th, (h->p.nz + zc - 1) / zc);
 }
 
 // partials of a stage launch, one per CTA
-long long stage_parts(const gpe_handle* h, int kind) {
+long long stage_parts(gpe_handle* h, int kind) {
   const dim3 g = stage_grid(h, kind);
   return (long long)g.x * g.y * g.z;
 }
 
-// Planes per CTA of every stage kernel the handle launches, chosen by the
-// kernel's CTAs per SM (the Cash-Karp stages with many point-wise inputs hold
-// half as many as the others).
-int choose_chunks(gpe_handle* h, int tile_zc) {
-  std::vector<int> kinds = {K_ENERGY};
-  switch (h->p.scheme) {
-    case GPE_EULER: kinds.insert(kinds.end(), {K_EULER}); break;
-    case GPE_RK2: kinds.insert(kinds.end(), {K_RK2_1, K_RK2_2}); break;
-    case GPE_RK4: kinds.insert(kinds.end(), {K_RK4_1, K_RK4_2, K_RK4_3, K_RK4_4}); break;
-    default: kinds.insert(kinds.end(), {K_CK_1, K_CK_2, K_CK_3, K_CK_4, K_CK_5, K_CK_6});
+// Make room for the partials of n blocks.
+int ensure_parts(gpe_handle* h, long long n) {
+  if (n <= h->part_cap) return GPE_OK;
+  if (h->part) {
+    CU(h, cudaStreamSynchronize(h->st));
+    cudaFree(h->part);
+    h->part = nullptr;
+    h->part_cap = 0;
   }
-  const int th = tile_rows(h->tma_ty);
-  const long long tiles = (long long)((h->p.nx + 31) / 32) * ((h->p.ny + th - 1) / th);
-  for (int k : kinds) {
-    if (tile_zc > 0) {
-      h->zck[k] = std::min(tile_zc, h->p.nz);
-    } else if (h->tma_ty == TILE_SITE) {
-      h->zck[k] = 1;
-    } else if (!h->use_tma) {
-      h->zck[k] = default_zc(h->g, th, h->esz);
-    } else {
-      int per = 0;
-      cudaError_t e = h->cmode == CM_F64   ? stage_tma_occupancy_f64(k, h->R, h->tma_ty, &per)
-                      : h->cmode == CM_F32 ? stage_tma_occupancy_f32(k, h->R, h->tma_ty, &per)
-                                           : stage_tma_occupancy_f32x(k, h->R, h->tma_ty, &per);
-      CU(h, e);
-      h->zck[k] = balanced_zc(h->g, h->esz, h->R, tiles, (long long)h->nsm * std::max(per, 1));
-    }
+  if (cudaMalloc(&h->part, n * RED_SLOTS * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(h, GPE_ERR_NOMEM, "out of device memory for the partials of a reduction");
   }
+  h->part_cap = n;
   return GPE_OK;
 }
 
 cudaError_t launch_raw(gpe_handle* h, int kind, const StageArgs& a_in) {
   StageArgs a = a_in;
   a.status = h->status;
-  a.zc = h->zck[kind];
+  a.zc = chunk_of(h, kind);
   const dim3 grid = stage_grid(h, kind);
   set_f32_constants(a);
   if (!h->use_tma || h->tma_ty == TILE_SITE) {
@@ -379,17 +391,15 @@ StageArgs base_args(gpe_handle* h) {
   return a;
 }
 
-int finalize_into(gpe_handle* h, const double* part, int slot, long long nparts) {
-  k_finalize<<<1, 256, 0, h->st>>>(part, nparts, h->dres + 3 * slot);
+int finalize_into(gpe_handle* h, int slot, long long nparts) {
+  k_finalize<<<1, 256, 0, h->st>>>(h->part, nparts, h->dres + 3 * slot);
   CU(h, cudaGetLastError());
   return GPE_OK;
 }
 
 // A stage kernel whose bounded mbarrier wait expired leaves a non-zero
 // status word; report it as GPE_ERR_TIMEOUT (and clear it).
-int check_status(gpe_handle* h) {
-  int st = 0;
-  CU(h, cudaMemcpy(&st, h->status, sizeof(int), cudaMemcpyDeviceToHost));
+int report_status(gpe_handle* h, int st) {
   if (st != 0) {
     CU(h, cudaMemset(h->status, 0, sizeof(int)));
     return fail(h, GPE_ERR_TIMEOUT, "a stage kernel's bounded wait for its TMA copies expired");
@@ -397,13 +407,30 @@ int check_status(gpe_handle* h) {
   return GPE_OK;
 }
 
-int fetch_results(gpe_handle* h) {
+int check_status(gpe_handle* h) {
+  int st = 0;
+  CU(h, cudaMemcpy(&st, h->status, sizeof(int), cudaMemcpyDeviceToHost));
+  return report_status(h, st);
+}
+
+// Queue the copy of the reductions and the status word to the host: one copy,
+// so a call waits for the device once.
+constexpr size_t RESULT_BYTES = 7 * sizeof(double);
+cudaError_t copy_results(gpe_handle* h) {
+  return cudaMemcpyAsync(h->hres, h->dres, RESULT_BYTES, cudaMemcpyDeviceToHost, h->st);
+}
+
+// Wait for the call's work and take its results; copied: the copy is queued
+// already (by the graph of a step with a norm).
+int fetch_results(gpe_handle* h, bool copied = false) {
   // z-slabs: norms and energies are sums over the slabs, errmax a maximum
   // (the MPI_ALLREDUCE of src/variables.f90:554-604, src/solve.f90:189-190)
   if (h->nccl && nccl_reduce_results(h->nccl, h->dres, h->st, h->xerr) != 0)
     return fail(h, GPE_ERR_CUDA, "z-slab reduction failed");
-  CU(h, cudaMemcpyAsync(h->hres, h->dres, 6 * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+  if (!copied) CU(h, copy_results(h));
   CU(h, cudaStreamSynchronize(h->st));
+  int st;
+  memcpy(&st, h->hres + 6, sizeof(st));
   if (h->prof) prof_resolve(h);
   if (h->hub && h->hub->n > 1) {
     SlabHub* hub = h->hub;
@@ -418,7 +445,7 @@ int fetch_results(gpe_handle* h) {
       return fail(h, GPE_ERR_TIMEOUT, "a z-slab of the hub stopped calling in (barrier timeout)");
     for (int q = 0; q < 6; ++q) h->hres[q] = v[q];
   }
-  return check_status(h);
+  return report_status(h, st);
 }
 
 double rk_param(double v, double def) { return v != 0.0 ? v : def; }
@@ -435,15 +462,21 @@ int enqueue_fixed_step(gpe_handle* h, double dr, double di, bool energy, bool no
   StageArgs a = base_args(h);
   void** F = h->fields.data();
   const int sc = h->p.scheme;
+  if (energy || norm) {
+    const int first = sc == GPE_RK4 ? K_RK4_1 : (sc == GPE_RK2 ? K_RK2_1 : K_EULER);
+    const int last = sc == GPE_RK4 ? K_RK4_4 : (sc == GPE_RK2 ? K_RK2_2 : K_EULER);
+    if (int rc = ensure_parts(h, std::max(energy ? stage_parts(h, first) : 0, norm ? stage_parts(h, last) : 0)))
+      return rc;
+  }
   if (sc == GPE_RK4) {
     void *psi = F[0], *A = F[1], *B = F[2], *Q = F[3];
     // s1: k1 = f(psi); A = psi + dt/2 k1
     a.in = psi; a.out = A;
     a.cf_r[0] = 0.5 * dr; a.cf_i[0] = 0.5 * di;
     a.want_energy = energy;
-    a.partials = energy ? h->part_a : nullptr;
+    a.partials = energy ? h->part : nullptr;
     CU(h, launch(h, K_RK4_1, a));
-    if (energy && finalize_into(h, h->part_a, 0, stage_parts(h, K_RK4_1))) return GPE_ERR_CUDA;
+    if (energy && finalize_into(h, 0, stage_parts(h, K_RK4_1))) return GPE_ERR_CUDA;
     a.want_energy = 0;
     a.partials = nullptr;
     // s2: k2 = f(A); B = psi + dt/2 k2; Q = (psi + A) + dt k2
@@ -459,9 +492,9 @@ int enqueue_fixed_step(gpe_handle* h, double dr, double di, bool energy, bool no
     a.in = A; a.psi = nullptr; a.out = psi;
     a.cf_r[0] = dr / 6.0; a.cf_i[0] = di / 6.0;
     a.want_norm = norm;
-    a.partials = norm ? h->part_b : nullptr;
+    a.partials = norm ? h->part : nullptr;
     CU(h, launch(h, K_RK4_4, a));
-    if (norm && finalize_into(h, h->part_b, 1, stage_parts(h, K_RK4_4))) return GPE_ERR_CUDA;
+    if (norm && finalize_into(h, 1, stage_parts(h, K_RK4_4))) return GPE_ERR_CUDA;
     return GPE_OK;
   }
   if (sc == GPE_RK2) {
@@ -469,16 +502,16 @@ int enqueue_fixed_step(gpe_handle* h, double dr, double di, bool energy, bool no
     a.in = psi; a.out = A;
     a.cf_r[0] = 0.5 * dr; a.cf_i[0] = 0.5 * di;
     a.want_energy = energy;
-    a.partials = energy ? h->part_a : nullptr;
+    a.partials = energy ? h->part : nullptr;
     CU(h, launch(h, K_RK2_1, a));
-    if (energy && finalize_into(h, h->part_a, 0, stage_parts(h, K_RK2_1))) return GPE_ERR_CUDA;
+    if (energy && finalize_into(h, 0, stage_parts(h, K_RK2_1))) return GPE_ERR_CUDA;
     a.want_energy = 0;
     a.in = A; a.psi = psi; a.out = psi;
     a.cf_r[0] = dr; a.cf_i[0] = di;
     a.want_norm = norm;
-    a.partials = norm ? h->part_b : nullptr;
+    a.partials = norm ? h->part : nullptr;
     CU(h, launch(h, K_RK2_2, a));
-    if (norm && finalize_into(h, h->part_b, 1, stage_parts(h, K_RK2_2))) return GPE_ERR_CUDA;
+    if (norm && finalize_into(h, 1, stage_parts(h, K_RK2_2))) return GPE_ERR_CUDA;
     return GPE_OK;
   }
   // Euler: new = old + dt f(old), written into the other buffer
@@ -488,13 +521,13 @@ int enqueue_fixed_step(gpe_handle* h, double dr, double di, bool energy, bool no
   a.want_energy = energy;
   a.want_norm = norm;
   if (energy && !norm) {
-    a.partials = h->part_a;
+    a.partials = h->part;
     CU(h, launch(h, K_EULER, a));
-    if (finalize_into(h, h->part_a, 0, stage_parts(h, K_EULER))) return GPE_ERR_CUDA;
+    if (finalize_into(h, 0, stage_parts(h, K_EULER))) return GPE_ERR_CUDA;
   } else {
-    a.partials = norm ? h->part_b : nullptr;
+    a.partials = norm ? h->part : nullptr;
     CU(h, launch(h, K_EULER, a));
-    if (norm && finalize_into(h, h->part_b, 1, stage_parts(h, K_EULER))) return GPE_ERR_CUDA;
+    if (norm && finalize_into(h, 1, stage_parts(h, K_EULER))) return GPE_ERR_CUDA;
     // one kernel produced both sums: move the energy into its slot
     if (energy) CU(h, cudaMemcpyAsync(h->dres + 1, h->dres + 4, sizeof(double), cudaMemcpyDeviceToDevice, h->st));
   }
@@ -517,6 +550,7 @@ int rk45_step(gpe_handle* h, gpe_step_info* io, bool energy, bool norm) {
   void* K[5] = {F[4], F[5], F[6], F[7], F[8]};
   double errmax = 0.0;
   bool first = true;
+  if (int rc = ensure_parts(h, std::max(stage_parts(h, K_CK_6), energy ? stage_parts(h, K_CK_1) : 0))) return rc;
   for (int attempt = 0;; ++attempt) {
     if (attempt > 10000) return fail(h, GPE_ERR_STATE, "rkqs: no acceptable step after 10000 attempts");
     StageArgs a = base_args(h);
@@ -541,11 +575,11 @@ int rk45_step(gpe_handle* h, gpe_step_info* io, bool energy, bool norm) {
         a.want_norm = norm;
       }
       a.want_energy = (m == 0 && energy && first);
-      a.partials = (m == 5) ? h->part_b : (a.want_energy ? h->part_a : nullptr);
+      a.partials = (m == 5 || a.want_energy) ? h->part : nullptr;
       CU(h, launch(h, K_CK_1 + m, a));
-      if (a.want_energy && finalize_into(h, h->part_a, 0, stage_parts(h, K_CK_1))) return GPE_ERR_CUDA;
+      if (a.want_energy && finalize_into(h, 0, stage_parts(h, K_CK_1))) return GPE_ERR_CUDA;
     }
-    if (finalize_into(h, h->part_b, 1, stage_parts(h, K_CK_6))) return GPE_ERR_CUDA;
+    if (finalize_into(h, 1, stage_parts(h, K_CK_6))) return GPE_ERR_CUDA;
     if (int rc = fetch_results(h)) return rc;
     first = false;
     errmax = h->hres[5] / eps;
@@ -583,14 +617,15 @@ int norm_now(gpe_handle* h, double* out) {
   const Geom& g = h->g;
   const size_t ntot = (size_t)h->p.nx + h->p.ny + h->p.nz;
   const double* w = h->tables + 2 * ntot;
+  if (int rc = ensure_parts(h, h->norm_npart)) return rc;
   if (h->esz == 16)
     k_norm<double2><<<h->norm_grid, dim3(32, 8), 0, h->st>>>((const double2*)h->fields[h->cur], g, h->zc, w,
-                                                             w + g.nx, w + g.nx + g.ny, h->part_b);
+                                                             w + g.nx, w + g.nx + g.ny, h->part);
   else
     k_norm<float2><<<h->norm_grid, dim3(32, 8), 0, h->st>>>((const float2*)h->fields[h->cur], g, h->zc, w,
-                                                            w + g.nx, w + g.nx + g.ny, h->part_b);
+                                                            w + g.nx, w + g.nx + g.ny, h->part);
   CU(h, cudaGetLastError());
-  if (int rc = finalize_into(h, h->part_b, 1, h->norm_npart)) return rc;
+  if (int rc = finalize_into(h, 1, h->norm_npart)) return rc;
   if (int rc = fetch_results(h)) return rc;
   *out = ((h->hres[3] * h->dx) * h->dy) * h->dz;
   return GPE_OK;
@@ -753,10 +788,6 @@ int create_impl(const gpe_params* p, const SlabSpec* sp, gpe_handle** out) {
     gpe_destroy(h);
     return fail(nullptr, rc, m);
   };
-  if (int rc = choose_chunks(h, p->tile_zc)) return bail(rc);
-  long long npart_alloc = h->norm_npart;
-  for (int k = 0; k < K_NUM; ++k)
-    if (h->zck[k]) npart_alloc = std::max(npart_alloc, stage_parts(h, k));
   if (sp && sp->hub) {
     h->hub = sp->hub;
     h->st = sp->hub->st;
@@ -784,25 +815,17 @@ int create_impl(const gpe_params* p, const SlabSpec* sp, gpe_handle** out) {
         return bail(GPE_ERR_CUDA);
       }
   }
-  if (cudaMalloc(&h->status, sizeof(int)) != cudaSuccess) {
-    cudaGetLastError();
-    h->err = "out of device memory (status word)";
-    return bail(GPE_ERR_NOMEM);
-  }
-  cudaMemsetAsync(h->status, 0, sizeof(int), h->st);
   std::vector<double> tab;
   build_tables(h, tab);
   if (cudaMalloc(&h->tables, tab.size() * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&h->part_a, npart_alloc * RED_SLOTS * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&h->part_b, npart_alloc * RED_SLOTS * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&h->dres, 6 * sizeof(double)) != cudaSuccess ||
-      cudaMallocHost(&h->hres, 6 * sizeof(double)) != cudaSuccess) {
+      cudaMalloc(&h->dres, RESULT_BYTES) != cudaSuccess || cudaMallocHost(&h->hres, RESULT_BYTES) != cudaSuccess) {
     cudaGetLastError();
     h->err = "out of memory allocating tables / reduction buffers";
     return bail(GPE_ERR_NOMEM);
   }
   cudaMemcpyAsync(h->tables, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, h->st);
-  cudaMemsetAsync(h->dres, 0, 6 * sizeof(double), h->st);
+  cudaMemsetAsync(h->dres, 0, RESULT_BYTES, h->st);
+  h->status = (int*)(h->dres + 6);
   if (cudaStreamSynchronize(h->st) != cudaSuccess) {
     h->err = "initialisation failed";
     return bail(GPE_ERR_CUDA);
@@ -889,12 +912,10 @@ void gpe_destroy(gpe_handle* h) {
   for (void* f : h->fields)
     if (f) cudaFree(f);
   if (h->tables) cudaFree(h->tables);
-  if (h->part_a) cudaFree(h->part_a);
-  if (h->part_b) cudaFree(h->part_b);
+  if (h->part) cudaFree(h->part);
   if (h->dres) cudaFree(h->dres);
   if (h->hres) cudaFreeHost(h->hres);
   if (h->staging) cudaFree(h->staging);
-  if (h->status) cudaFree(h->status);
   if (h->fft_work) cudaFree(h->fft_work);
   for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
   for (cudaGraphExec_t g : h->step_graph)
@@ -970,8 +991,8 @@ int gpe_get_state_device(gpe_handle* h, void* psi_dev, int32_t dtype) {
 }
 
 // Graph of one (which = 0) or GRAPH_STEPS (1) fixed steps for the current dt,
-// captured on first use and whenever dt changes.  Only for schemes that keep
-// psi in place.
+// or of one with the norm and the results' copy (2), captured on first use and
+// whenever dt changes.  Only for schemes that keep psi in place.
 constexpr int GRAPH_STEPS = 8;
 static int ensure_step_graph(gpe_handle* h, int which, double dr, double di) {
   if (h->graph_dr != dr || h->graph_di != di) {
@@ -987,7 +1008,9 @@ static int ensure_step_graph(gpe_handle* h, int which, double dr, double di) {
   CU(h, cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
   h->capturing = true;
   int rc = GPE_OK;
-  for (int s = 0; s < (which ? GRAPH_STEPS : 1) && rc == GPE_OK; ++s) rc = enqueue_fixed_step(h, dr, di, false, false);
+  for (int s = 0; s < (which == 1 ? GRAPH_STEPS : 1) && rc == GPE_OK; ++s)
+    rc = enqueue_fixed_step(h, dr, di, false, which == 2);
+  if (rc == GPE_OK && which == 2 && copy_results(h) != cudaSuccess) rc = fail(h, GPE_ERR_CUDA, "capture failed");
   h->capturing = false;
   const cudaError_t e = cudaStreamEndCapture(h->st, &g);
   if (rc != GPE_OK) {
@@ -1029,7 +1052,10 @@ static int step_impl(gpe_handle* h, int64_t nsteps, gpe_step_info* io, bool wait
     // steps without reductions replay a captured graph (one launch instead of
     // one per stage); the first step of a call runs plainly, so every kernel
     // has been loaded and configured before any capture
-    const bool graphs = use_step_graphs(h) && nsteps >= 3;
+    // (a step with a norm from its second use on: a relaxation asks for one
+    // per call)
+    const bool can = use_step_graphs(h), graphs = can && nsteps >= 3;
+    bool copied = false;
     for (int64_t s = 0; s < nsteps;) {
       const bool e = want_e && s == 0, n = want_n && s == nsteps - 1;
       int64_t took = 1;
@@ -1039,6 +1065,10 @@ static int step_impl(gpe_handle* h, int64_t nsteps, gpe_step_info* io, bool wait
         if (int rc = ensure_step_graph(h, which, dr, di)) return rc;
         CU(h, cudaGraphLaunch(h->step_graph[which], h->st));
         if (which) took = GRAPH_STEPS;
+      } else if (can && n && !e && h->norm_steps++ > 0) {
+        if (int rc = ensure_step_graph(h, 2, dr, di)) return rc;
+        CU(h, cudaGraphLaunch(h->step_graph[2], h->st));
+        copied = true;
       } else if (int rc = enqueue_fixed_step(h, dr, di, e, n)) {
         return rc;
       }
@@ -1051,7 +1081,7 @@ static int step_impl(gpe_handle* h, int64_t nsteps, gpe_step_info* io, bool wait
       io->accepted += took;
     }
     if (!wait) return GPE_OK;
-    if (int rc = fetch_results(h)) return rc;
+    if (int rc = fetch_results(h, copied)) return rc;
   }
   if (want_e && nsteps > 0) io->energy = ((h->hres[1] * h->dx) * h->dy) * h->dz;
   if (want_n && nsteps > 0) {
@@ -1192,9 +1222,10 @@ int gpe_energy(gpe_handle* h, double* energy) {
   StageArgs a = base_args(h);
   a.in = h->fields[h->cur];
   a.want_energy = 1;
-  a.partials = h->part_a;
+  if (int rc = ensure_parts(h, stage_parts(h, K_ENERGY))) return rc;
+  a.partials = h->part;
   CU(h, launch(h, K_ENERGY, a));
-  if (int rc = finalize_into(h, h->part_a, 0, stage_parts(h, K_ENERGY))) return rc;
+  if (int rc = finalize_into(h, 0, stage_parts(h, K_ENERGY))) return rc;
   if (int rc = fetch_results(h)) return rc;
   *energy = ((h->hres[1] * h->dx) * h->dy) * h->dz;
   return GPE_OK;
@@ -1285,8 +1316,8 @@ int gpe_renormalise(gpe_handle* h, double norm) {
   if (!h || !(norm > 0)) return fail(h, GPE_ERR_BADARG, "norm must be > 0");
   CU(h, cudaSetDevice(h->dev));
   const double a = sqrt(h->p.nn), b = sqrt(norm);
-  if (h->esz == 16) k_scale<double2><<<148 * 8, 256, 0, h->st>>>((double2*)h->fields[h->cur], h->nelem, a, b);
-  else k_scale<float2><<<148 * 8, 256, 0, h->st>>>((float2*)h->fields[h->cur], h->nelem, a, b);
+  if (h->esz == 16) k_scale<double2><<<ROW_GRID, ROW_THREADS, 0, h->st>>>((double2*)h->fields[h->cur], h->nelem, a, b);
+  else k_scale<float2><<<ROW_GRID, ROW_THREADS, 0, h->st>>>((float2*)h->fields[h->cur], h->nelem, a, b);
   CU(h, cudaGetLastError());
   CU(h, cudaStreamSynchronize(h->st));
   return GPE_OK;
