@@ -108,6 +108,44 @@ __global__ void __launch_bounds__(256) k_norm(const S* __restrict__ f, Geom g, i
   block_reduce_store<256>(s, 0.0, 0.0, partials);
 }
 
+// get_norm of many solves in one launch: block b sums the planes k0 ..
+// k0 + NORM_PLANES - 1 of solve items[b].solve, rows to warps in a fixed order.
+// The partition depends on the solve's own grid only, so a solve's norm does
+// not depend on what else is in the batch or on the stage launches' items.
+struct NormSolve {
+  Geom g;
+  const double *wx, *wy, *wz;
+  const void* psi;
+};
+struct NormItem {
+  int solve, k0;
+};
+constexpr int NORM_PLANES = 4;
+
+template <class S>
+__global__ void __launch_bounds__(ROW_THREADS) k_norm_batch(const NormSolve* __restrict__ sv,
+                                                            const NormItem* __restrict__ items, double* partials) {
+  const NormItem it = items[blockIdx.x];
+  const NormSolve n = sv[it.solve];
+  const Geom g = n.g;
+  const int lane = threadIdx.x & 31;
+  const int rows = min(NORM_PLANES, g.nz - it.k0) * g.ny;
+  double s = 0.0;
+  for (int r = threadIdx.x >> 5; r < rows; r += ROW_THREADS / 32) {
+    const int dk = r / g.ny, j = r - dk * g.ny, k = it.k0 + dk;
+    const S* row = (const S*)n.psi + (long long)(k + 2) * g.pz + (long long)(j + 2) * g.px + g.xoff;
+    double t = 0.0;
+#pragma unroll 4
+    for (int i = lane; i < g.nx; i += 32) {
+      const S v = row[i];
+      const double vr = (double)v.x, vi = (double)v.y;
+      t += n.wx[i] * (vr * vr + vi * vi);
+    }
+    s += (n.wy[j] * n.wz[k]) * t;
+  }
+  block_reduce_store_at<ROW_THREADS>(s, 0.0, 0.0, partials, blockIdx.x);
+}
+
 // Sum (slots 0,1) and max (slot 2) of nb block partials in a fixed order.
 static __global__ void __launch_bounds__(256) k_finalize(const double* __restrict__ partials, long long nb, double* out) {
   __shared__ double s0[256], s1[256], s2[256];

@@ -6,8 +6,10 @@
 // are grouped into classes by (storage/compute mode, scheme family); each
 // class keeps a work list of (solve, tile, z-chunk) items and a device table
 // of per-solve stage arguments and tensor maps.  One persistent launch of
-// k_stage_batch per Runge-Kutta stage advances every solve of a class; the
-// RK4 step of a class is captured once into a CUDA graph and replayed.
+// k_stage_batch per Runge-Kutta stage advances every solve of a class, each
+// class on its own stream, the host taking the classes step by step in turn.
+// (Replayed step graphs kept the host in the launch of a class's next step
+// until the one before it was done, so the classes ran one after another.)
 // RKF45 solves share their attempts: after each attempt every solve's error
 // norm is read back and that solve alone accepts or rejects (rkqs,
 // src/solve.f90:158-244), so per-solve time steps diverge freely.
@@ -160,6 +162,8 @@ struct HostPinned {
   }
 };
 
+constexpr int QUEUE_STEPS = 64;  // RK4 steps a class's queue counters are zeroed for at once
+
 struct Class {
   std::vector<Solve*> solves;
   bool dirty = true;
@@ -173,6 +177,16 @@ struct Class {
   HostPinned<BatchStage> htab;
   HostPinned<double> hres;
   HostPinned<int> hstatus;  // device status word after the class's last RKF45 attempt
+  // norms of the class's solves (k_norm_batch), formed once per pool step
+  DevBuf<NormSolve> nsolve;
+  HostPinned<NormSolve> hnsolve;
+  DevBuf<NormItem> nitem;
+  DevBuf<int> nfirst;
+  DevBuf<double> npart, nres;
+  HostPinned<double> hnres;
+  std::vector<Solve*> norm_for;  // the solves the norm's work list was built for
+  std::vector<NormItem> hnitem;
+  std::vector<int> hnfirst;
   std::vector<BatchItem> hitems;
   std::vector<int> horder;
   // the solves (in order) the device work list was built for; an RKF45 class
@@ -180,19 +194,7 @@ struct Class {
   std::vector<Solve*> built_for;
   std::vector<int> hfirst;
   int nitems = 0;
-  // RK4 step graphs: without reductions, and with the per-solve norm (the
-  // last step of a chunk)
-  cudaGraph_t graph = nullptr, graph_n = nullptr;
-  cudaGraphExec_t gexec = nullptr, gexec_n = nullptr;
   cudaStream_t st = nullptr;  // classes run concurrently, one stream each
-  void drop_graph() {
-    if (gexec) cudaGraphExecDestroy(gexec);
-    if (graph) cudaGraphDestroy(graph);
-    if (gexec_n) cudaGraphExecDestroy(gexec_n);
-    if (graph_n) cudaGraphDestroy(graph_n);
-    gexec = gexec_n = nullptr;
-    graph = graph_n = nullptr;
-  }
 };
 
 double now_s(const std::chrono::steady_clock::time_point& t0) {
@@ -335,7 +337,6 @@ void rk4_tables(gpe_pool* P, Solve* s, BatchStage* t4) {
   b = make_stage(P, s, K_RK4_4, 1, 0, {3});
   b.args.acc = s->f[3];
   b.args.cf_r[0] = dr / 6.0; b.args.cf_i[0] = di / 6.0;
-  b.args.want_norm = 1;
   t4[3] = b;
 }
 
@@ -367,14 +368,54 @@ void rk45_tables(gpe_pool* P, Solve* s, BatchStage* t6) {
       b.args.dte_r = s->dte_r;
       b.args.dte_i = s->dte_i;
       b.args.inv_adt = 1.0 / hypot(s->dr, s->di);
-      b.args.want_norm = 1;
     }
     t6[m] = b;
   }
 }
 
+// z planes per work item of the class's solves (those without a chosen
+// tile_zc): as long as the items still fill the device.
+// An item costs its planes and about 3R more (queue fill, halo planes), so
+// long items are cheaper where there is work for every slot -- the uneven mix
+// of 64 solves of 32^3-160^3 wants 64 planes, 44.2 G site-updates/s against
+// 42.8 with 16 and 32 -- but a launch is never shorter than its longest item:
+// 16 solves of 32^3-128^3 in five classes took 16.0 ms for 40 steps with
+// items of up to 64 planes (46 to 132 of them in a launch for 592 slots) and
+// take 9.2 so; one 96^3 solve runs at 17 instead of 3.5 G site-updates/s.
+// States do not depend on the items.
+void choose_items(int cm, int fam, const std::vector<Solve*>& sv) {
+  int occ = 0;
+  BatchLaunch q{};
+  q.ns = (int)sv.size();
+  launch_batch(cm, fam == FAM_RK45 ? K_CK_4 : K_RK4_2, 0, nullptr, q, &occ);
+  const double slots = std::max(1, occ);
+  const int lead = 3 * class_radius(cm);
+  int best = 64;
+  double best_t = 0.0;
+  for (int z = 64; z >= 2; z = z > 16 ? z - 8 : z - 1) {
+    double work = 0.0, longest = 0.0;
+    for (const Solve* s : sv) {
+      const int zc = s->p.tile_zc > 0 ? std::min(s->p.tile_zc, s->g.nz) : std::min(s->g.nz, z);
+      const int n = (s->g.nz + zc - 1) / zc;
+      work += (double)s->ntx * s->nty * (s->g.nz + (double)n * lead);
+      longest = std::max(longest, (double)zc + lead);
+    }
+    const double t = std::max(longest, work / slots + 0.1 * longest);
+    if (best_t == 0.0 || t < best_t) {
+      best = z;
+      best_t = t;
+    }
+  }
+  for (Solve* s : sv) {
+    s->zc = s->p.tile_zc > 0 ? std::min(s->p.tile_zc, s->g.nz) : std::min(s->g.nz, best);
+    s->ntz = (s->g.nz + s->zc - 1) / s->zc;
+  }
+}
+
 // Work list of the given solves (in order) into the class buffers.
-int build_items(gpe_pool* P, Class& c, const std::vector<Solve*>& sv) {
+int build_items(gpe_pool* P, int cm, int fam, const std::vector<Solve*>& sv) {
+  Class& c = P->cls[cm][fam];
+  choose_items(cm, fam, sv);
   c.built_for = sv;
   c.hitems.clear();
   c.hfirst.assign(1, 0);
@@ -400,7 +441,7 @@ int build_items(gpe_pool* P, Class& c, const std::vector<Solve*>& sv) {
   std::stable_sort(c.horder.begin(), c.horder.end(), [&](int u, int v) { return cost[u] > cost[v]; });
   PCU(P, c.items.ensure(c.hitems.size()));
   PCU(P, c.order.ensure(c.horder.size()));
-  PCU(P, c.queue.ensure(8));
+  PCU(P, c.queue.ensure(4 * QUEUE_STEPS));
   PCU(P, c.first.ensure(c.hfirst.size()));
   PCU(P, c.part.ensure(c.hitems.size() * RED_SLOTS));
   PCU(P, c.res.ensure(sv.size() * RED_SLOTS));
@@ -427,75 +468,91 @@ int ensure_stream(gpe_pool* P, Class& c) {
   return GPE_OK;
 }
 
-// Capture one RK4 step of a class: the queue reset and four batched
-// launches; with_norm: stage 4 reads table row 3 (norm on) and writes the
-// partials, else row 4 (norm off) and no partials.
-int capture_rk4_step(gpe_pool* P, Class& c, int cm, int ns, const int* grids, bool with_norm,
-                     cudaGraph_t* graph, cudaGraphExec_t* gexec) {
-  const int kinds[4] = {K_RK4_1, K_RK4_2, K_RK4_3, K_RK4_4};
-  PCU(P, cudaStreamBeginCapture(c.st, cudaStreamCaptureModeThreadLocal));
-  cudaError_t e = cudaMemsetAsync(c.queue.p, 0, 4 * sizeof(int), c.st);
-  for (int m = 0; m < 4 && e == cudaSuccess; ++m) {
-    const int row = (m == 3 && !with_norm) ? 4 : m;
-    e = launch_batch(cm, kinds[m], grids[m], c.st,
-                     BatchLaunch{c.tab.p + (size_t)row * ns, c.htab.p + (size_t)row * ns, ns, c.items.p, c.order.p,
-                                 c.nitems, c.queue.p + m, (m == 3 && with_norm) ? c.part.p : nullptr},
-                     nullptr);
+// Queue the norms of the class's solves (their current states) on its stream.
+int norms_enqueue(gpe_pool* P, int cm, int fam) {
+  Class& c = P->cls[cm][fam];
+  const int ns = (int)c.solves.size();
+  if (int rc = ensure_stream(P, c)) return rc;
+  PCU(P, c.nsolve.ensure(ns));
+  PCU(P, c.hnsolve.ensure(ns));
+  PCU(P, c.nres.ensure((size_t)ns * RED_SLOTS));
+  PCU(P, c.hnres.ensure((size_t)ns * RED_SLOTS));
+  if (c.norm_for != c.solves) {
+    PCU(P, cudaStreamSynchronize(c.st));
+    c.hnitem.clear();
+    c.hnfirst.assign(1, 0);
+    for (int q = 0; q < ns; ++q) {
+      for (int k = 0; k < c.solves[q]->g.nz; k += NORM_PLANES) c.hnitem.push_back(NormItem{q, k});
+      c.hnfirst.push_back((int)c.hnitem.size());
+    }
+    PCU(P, c.nitem.ensure(c.hnitem.size()));
+    PCU(P, c.nfirst.ensure(c.hnfirst.size()));
+    PCU(P, c.npart.ensure(c.hnitem.size() * RED_SLOTS));
+    PCU(P, cudaMemcpyAsync(c.nitem.p, c.hnitem.data(), c.hnitem.size() * sizeof(NormItem), cudaMemcpyHostToDevice,
+                           c.st));
+    PCU(P, cudaMemcpyAsync(c.nfirst.p, c.hnfirst.data(), c.hnfirst.size() * sizeof(int), cudaMemcpyHostToDevice,
+                           c.st));
+    c.norm_for = c.solves;
   }
-  cudaGraph_t g = nullptr;
-  cudaError_t e2 = cudaStreamEndCapture(c.st, &g);
-  if (e != cudaSuccess || e2 != cudaSuccess) {
-    if (g) cudaGraphDestroy(g);
-    return pfail(P, GPE_ERR_CUDA, std::string("capturing the batched RK4 step failed: ") +
-                                      cudaGetErrorString(e != cudaSuccess ? e : e2));
+  for (int q = 0; q < ns; ++q) {
+    const Solve* s = c.solves[q];
+    const double* w = s->tables + 2 * ((size_t)s->g.nx + s->g.ny + s->g.nz);
+    c.hnsolve.p[q] = NormSolve{s->g, w, w + s->g.nx, w + s->g.nx + s->g.ny, s->f[s->cur]};
   }
-  *graph = g;
-  PCU(P, cudaGraphInstantiate(gexec, g, 0));
+  PCU(P, cudaMemcpyAsync(c.nsolve.p, c.hnsolve.p, ns * sizeof(NormSolve), cudaMemcpyHostToDevice, c.st));
+  const int nb = (int)c.hnitem.size();
+  if (class_cmode(cm) == CM_F64) k_norm_batch<double2><<<nb, ROW_THREADS, 0, c.st>>>(c.nsolve.p, c.nitem.p, c.npart.p);
+  else k_norm_batch<float2><<<nb, ROW_THREADS, 0, c.st>>>(c.nsolve.p, c.nitem.p, c.npart.p);
+  k_finalize_ranges<<<ns, 256, 0, c.st>>>(c.npart.p, c.nfirst.p, c.nres.p);
+  PCU(P, cudaGetLastError());
+  PCU(P, cudaMemcpyAsync(c.hnres.p, c.nres.p, (size_t)ns * RED_SLOTS * sizeof(double), cudaMemcpyDeviceToHost, c.st));
   return GPE_OK;
 }
 
-// Enqueue `chunk` RK4 steps of every solve of an RK4 class on the class's
-// stream (each step a captured graph of four batched launches; only the last
-// one forms the per-solve norm of the result), then the norm's finalisation;
-// returns without waiting.
-int rk4_enqueue(gpe_pool* P, int cm, int64_t chunk) {
+double norm_of(const Class& c, int q) {
+  const Solve* s = c.solves[q];
+  return ((c.hnres.p[q * RED_SLOTS + RED_NORM] * s->d[0]) * s->d[1]) * s->d[2];
+}
+
+// Work list and stage tables of an RK4 class whose solves changed.
+int rk4_prepare(gpe_pool* P, int cm) {
   Class& c = P->cls[cm][FAM_RK4];
   const int ns = (int)c.solves.size();
   if (int rc = ensure_stream(P, c)) return rc;
-  if (c.dirty) {
-    c.drop_graph();
-    PCU(P, cudaStreamSynchronize(c.st));
-    if (int rc = build_items(P, c, c.solves)) return rc;
-    // table rows: stages 1-4, then stage 4 without the norm
-    PCU(P, c.tab.ensure((size_t)5 * ns));
-    PCU(P, c.htab.ensure((size_t)5 * ns));
-    std::vector<BatchStage> t4(4);
-    for (int q = 0; q < ns; ++q) {
-      rk4_tables(P, c.solves[q], t4.data());
-      for (int m = 0; m < 4; ++m) c.htab.p[(size_t)m * ns + q] = t4[m];
-      BatchStage b = t4[3];
-      b.args.want_norm = 0;
-      c.htab.p[(size_t)4 * ns + q] = b;
-    }
-    for (size_t r = 0; r < (size_t)5 * ns; ++r) set_f32_constants(c.htab.p[r].args);
-    PCU(P, cudaMemcpyAsync(c.tab.p, c.htab.p, (size_t)5 * ns * sizeof(BatchStage), cudaMemcpyHostToDevice, c.st));
-    const int kinds[4] = {K_RK4_1, K_RK4_2, K_RK4_3, K_RK4_4};
-    int grids[4];
-    for (int m = 0; m < 4; ++m) grids[m] = grid_for(cm, kinds[m], c.nitems, ns);
-    PCU(P, cudaStreamSynchronize(c.st));
-    if (int rc = capture_rk4_step(P, c, cm, ns, grids, false, &c.graph, &c.gexec)) return rc;
-    if (int rc = capture_rk4_step(P, c, cm, ns, grids, true, &c.graph_n, &c.gexec_n)) return rc;
-    c.dirty = false;
+  if (!c.dirty) return GPE_OK;
+  PCU(P, cudaStreamSynchronize(c.st));
+  if (int rc = build_items(P, cm, FAM_RK4, c.solves)) return rc;
+  PCU(P, c.tab.ensure((size_t)4 * ns));
+  PCU(P, c.htab.ensure((size_t)4 * ns));
+  std::vector<BatchStage> t4(4);
+  for (int q = 0; q < ns; ++q) {
+    rk4_tables(P, c.solves[q], t4.data());
+    for (int m = 0; m < 4; ++m) c.htab.p[(size_t)m * ns + q] = t4[m];
   }
-  for (int64_t q = 0; q + 1 < chunk; ++q) PCU(P, cudaGraphLaunch(c.gexec, c.st));
-  if (chunk > 0) PCU(P, cudaGraphLaunch(c.gexec_n, c.st));
-  k_finalize_ranges<<<ns, 256, 0, c.st>>>(c.part.p, c.first.p, c.res.p);
-  PCU(P, cudaGetLastError());
-  PCU(P, cudaMemcpyAsync(c.hres.p, c.res.p, (size_t)ns * RED_SLOTS * sizeof(double), cudaMemcpyDeviceToHost, c.st));
+  for (size_t r = 0; r < (size_t)4 * ns; ++r) set_f32_constants(c.htab.p[r].args);
+  PCU(P, cudaMemcpyAsync(c.tab.p, c.htab.p, (size_t)4 * ns * sizeof(BatchStage), cudaMemcpyHostToDevice, c.st));
+  PCU(P, cudaStreamSynchronize(c.st));
+  c.dirty = false;
   return GPE_OK;
 }
 
-// After rk4_enqueue's work completed: advance the solves' clocks.
+// Enqueue step q of a call for every solve of an RK4 class: four batched
+// launches on the class's stream.  Their queue counters are zeroed for
+// QUEUE_STEPS steps at a time.
+int rk4_step(gpe_pool* P, int cm, int64_t q) {
+  Class& c = P->cls[cm][FAM_RK4];
+  const int ns = (int)c.solves.size(), at = (int)(q % QUEUE_STEPS);
+  const int kinds[4] = {K_RK4_1, K_RK4_2, K_RK4_3, K_RK4_4};
+  if (at == 0) PCU(P, cudaMemsetAsync(c.queue.p, 0, 4 * QUEUE_STEPS * sizeof(int), c.st));
+  for (int m = 0; m < 4; ++m)
+    PCU(P, launch_batch(cm, kinds[m], grid_for(cm, kinds[m], c.nitems, ns), c.st,
+                        BatchLaunch{c.tab.p + (size_t)m * ns, c.htab.p + (size_t)m * ns, ns, c.items.p, c.order.p,
+                                    c.nitems, c.queue.p + 4 * at + m, nullptr},
+                        nullptr));
+  return GPE_OK;
+}
+
+// After the steps' work completed: advance the solves' clocks.
 int rk4_collect(gpe_pool* P, int cm, int64_t chunk) {
   Class& c = P->cls[cm][FAM_RK4];
   PCU(P, cudaStreamSynchronize(c.st));
@@ -507,7 +564,7 @@ int rk4_collect(gpe_pool* P, int cm, int64_t chunk) {
     }
     s->p_index += chunk;
     s->done += chunk;
-    s->norm = ((c.hres.p[q * RED_SLOTS + 0] * s->d[0]) * s->d[1]) * s->d[2];
+    s->norm = norm_of(c, (int)q);
     if (!std::isfinite(s->norm)) s->status = GPE_ERR_NONFINITE;
   }
   return GPE_OK;
@@ -524,7 +581,7 @@ int rk45_enqueue(gpe_pool* P, int cm, std::vector<Solve*>& sv) {
   if (int rc = ensure_stream(P, c)) return rc;
   const int ns = (int)sv.size();
   if (c.dirty || sv != c.built_for) {
-    if (int rc = build_items(P, c, sv)) return rc;
+    if (int rc = build_items(P, cm, FAM_RK45, sv)) return rc;
     c.dirty = false;
   }
   PCU(P, c.tab.ensure((size_t)6 * ns));
@@ -604,7 +661,6 @@ int rk45_collect(gpe_pool* P, int cm, const std::vector<Solve*>& sv) {
     s->quota -= 1;
     s->dte_r = s->dr;  // next step's psi_scal uses the dt at rkqs entry
     s->dte_i = s->di;
-    s->norm = ((c.hres.p[q * RED_SLOTS + 0] * s->d[0]) * s->d[1]) * s->d[2];
   }
   return GPE_OK;
 }
@@ -674,16 +730,9 @@ static int pool_submit_impl(gpe_pool* P, const gpe_params* prm, const void* psi0
   s->cmode = cmode_of(*prm);
   s->fam = prm->scheme == GPE_RK45 ? FAM_RK45 : FAM_RK4;
   s->nf = scheme_fields(prm->scheme);
-  // z planes per work item: the caller's (autotuned) choice, else a batch
-  // default of up to 64 planes.  In a batch the other solves fill the GPU,
-  // so items can be long (fewer z-halo re-reads and queue fills per plane)
-  // instead of many: on the uneven 32^3-160^3 mix 64 beats 32, 48, 96 and
-  // 128 (44.2 against 42.1-43.8 G site-updates/s).
-  s->zc = prm->tile_zc > 0 ? std::min(prm->tile_zc, prm->nz) : std::min(prm->nz, 64);
   s->tile_h = batch_rows(s->cmode, s->fam);
   s->ntx = (prm->nx + 31) / 32;
   s->nty = (prm->ny + s->tile_h - 1) / s->tile_h;
-  s->ntz = (prm->nz + s->zc - 1) / s->zc;
   s->field_bytes = Arena::round((size_t)padded_elems(s->g) * s->esz);
   s->bytes = s->field_bytes * s->nf + Arena::round(tables_bytes(*prm));
   if (!P->alloc.alloc(s->bytes, &s->off)) {
@@ -764,10 +813,20 @@ int gpe_pool_step(gpe_pool* P, int64_t max_steps, int32_t* n_active) {
     int64_t chunk = max_steps;
     for (Solve* s : c.solves) chunk = std::min(chunk, s->nsteps - s->done);
     if (!c.solves.empty() && chunk > 0) {
-      if (int rc = rk4_enqueue(P, cm, chunk)) return rc;
+      if (int rc = rk4_prepare(P, cm)) return rc;
       chunks[cm] = chunk;
     }
   }
+  // step by step over the classes, so that each class's stream has work while
+  // the host is busy with the others
+  const int64_t longest = *std::max_element(chunks, chunks + NCLS);
+  for (int64_t q = 0; q < longest; ++q)
+    for (int cm = 0; cm < NCLS; ++cm)
+      if (q < chunks[cm])
+        if (int rc = rk4_step(P, cm, q)) return rc;
+  for (int cm = 0; cm < NCLS; ++cm)
+    if (chunks[cm])
+      if (int rc = norms_enqueue(P, cm, FAM_RK4)) return rc;
   for (int cm = 0; cm < NCLS; ++cm)
     for (Solve* s : P->cls[cm][FAM_RK45].solves) {
       s->quota = std::min(max_steps, s->nsteps - s->done);
@@ -785,6 +844,16 @@ int gpe_pool_step(gpe_pool* P, int64_t max_steps, int32_t* n_active) {
     for (int cm = 0; cm < NCLS; ++cm)
       if (!sv[cm].empty())
         if (int rc = rk45_collect(P, cm, sv[cm])) return rc;
+  }
+  for (int cm = 0; cm < NCLS; ++cm)
+    if (!P->cls[cm][FAM_RK45].solves.empty())
+      if (int rc = norms_enqueue(P, cm, FAM_RK45)) return rc;
+  for (int cm = 0; cm < NCLS; ++cm) {
+    Class& c = P->cls[cm][FAM_RK45];
+    if (c.solves.empty()) continue;
+    PCU(P, cudaStreamSynchronize(c.st));
+    for (size_t q = 0; q < c.solves.size(); ++q)
+      if (c.solves[q]->done > 0) c.solves[q]->norm = norm_of(c, (int)q);
   }
   for (int cm = 0; cm < NCLS; ++cm)
     if (chunks[cm])
@@ -839,6 +908,9 @@ int gpe_pool_step(gpe_pool* P, int64_t max_steps, int32_t* n_active) {
       if (retired) {
         c.solves.swap(keep);
         c.dirty = true;
+        // (a later solve may be given a retired one's address)
+        c.norm_for.clear();
+        c.built_for.clear();
       }
       active += (int)c.solves.size();
     }
@@ -892,7 +964,6 @@ void gpe_pool_destroy(gpe_pool* P) {
     for (int fam = 0; fam < NFAM; ++fam) {
       Class& c = P->cls[cm][fam];
       for (Solve* s : c.solves) delete s;
-      c.drop_graph();
       if (c.st) {
         cudaStreamSynchronize(c.st);
         cudaStreamDestroy(c.st);
@@ -907,6 +978,13 @@ void gpe_pool_destroy(gpe_pool* P) {
       c.htab.free();
       c.hres.free();
       c.hstatus.free();
+      c.nsolve.free();
+      c.hnsolve.free();
+      c.nitem.free();
+      c.nfirst.free();
+      c.npart.free();
+      c.nres.free();
+      c.hnres.free();
     }
   if (P->arena) cudaFree(P->arena);
   if (P->d_status) cudaFree(P->d_status);

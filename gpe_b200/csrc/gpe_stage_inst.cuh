@@ -212,7 +212,7 @@ __host__ __device__ constexpr bool is_rk4_kind(int k) {
 
 // Opt the batched kernel into its dynamic shared memory once per device and
 // cache how many of its CTAs fit on the device at once.
-template <class S, class C, int K, int TY, bool PAIR, int RR, bool PARG = false>
+template <class S, class C, int K, int TY, bool PAIR, int RR, int PARG>
 static cudaError_t batch_setup(int* occupancy) {
   using LY = TmaLayout<S, RR, StageTraits<K>::NPW, TY>;
   static unsigned long long done = 0;
@@ -236,64 +236,54 @@ static cudaError_t batch_setup(int* occupancy) {
   return cudaSuccess;
 }
 
-// One launch; with at most BATCH_PARAM_SOLVES solves their stage arguments
-// go into the launch's parameter space (the PARG kernel), else the kernel
-// reads them from the device table.  FP32 Cash-Karp stages keep the table
-// path: their item bodies read the arguments so often per site that
-// constant-cache reads cost more than the registers they free (a batch of
-// 16 FP32 RKF45 solves: 9.8 against 10.5 G accepted site-updates/s; FP64
-// Cash-Karp gains 14 %, the RK4 stages 4 %).
-template <class S, class C, int K, int TY, bool PAIR, int RR>
-static cudaError_t launch_batch_one(int grid, cudaStream_t st, const BatchLaunch& b) {
+template <class S, class C, int K, int TY, bool PAIR, int RR, int PARG>
+static cudaError_t launch_batch_rows(int grid, cudaStream_t st, const BatchLaunch& b) {
   using LY = TmaLayout<S, RR, StageTraits<K>::NPW, TY>;
   const dim3 block = PAIR ? dim3(16, 8) : dim3(32, TY / BATCH_PY);
-  constexpr bool kParamArgs = !(sizeof(C) == sizeof(float) && K >= K_CK_1 && K <= K_CK_6);
-  if constexpr (kParamArgs) {
-    if (b.htab && b.ns >= 1 && b.ns <= BATCH_PARAM_SOLVES) {
-      cudaError_t e = batch_setup<S, C, K, TY, PAIR, RR, true>(nullptr);
-      if (e != cudaSuccess) return e;
-      thread_local std::unique_ptr<BatchArgs> pa;  // 32 KB staging, copied by the launch
-      if (!pa) pa.reset(new BatchArgs);
-      for (int q = 0; q < b.ns; ++q) pa->a[q] = b.htab[q].args;
-      k_stage_batch<S, C, K, TY, BATCH_PY, PAIR, RR, true>
-          <<<grid, block, LY::SMEM, st>>>(b.tab, b.items, b.order, b.nitems, b.queue, b.partials, *pa);
-      return cudaGetLastError();
-    }
-  }
-  cudaError_t e = batch_setup<S, C, K, TY, PAIR, RR, false>(nullptr);
+  cudaError_t e = batch_setup<S, C, K, TY, PAIR, RR, PARG>(nullptr);
   if (e != cudaSuccess) return e;
-  k_stage_batch<S, C, K, TY, BATCH_PY, PAIR, RR, false>
-      <<<grid, block, LY::SMEM, st>>>(b.tab, b.items, b.order, b.nitems, b.queue, b.partials, NoBatchArgs{});
+  thread_local std::unique_ptr<BatchArgs<PARG>> pa;  // staging, copied by the launch
+  if (!pa) pa.reset(new BatchArgs<PARG>);
+  if constexpr (PARG > 0)
+    for (int q = 0; q < b.ns; ++q) pa->a[q] = b.htab[q].args;
+  k_stage_batch<S, C, K, TY, BATCH_PY, PAIR, RR, PARG>
+      <<<grid, block, LY::SMEM, st>>>(b.tab, b.items, b.order, b.nitems, b.queue, b.partials, *pa);
   return cudaGetLastError();
 }
 
-// CTAs of the kernel launch_batch_one would launch for b that fit on the
-// device at once (b.ns picks the parameter-space or the table kernel).
+// One launch (grid > 0), or the CTAs of its kernel that fit on the device at
+// once (grid <= 0).  With at most BATCH_PARAM_SOLVES solves their stage
+// arguments go into the launch's parameter space, else the kernel reads them
+// from the device table.  FP32 Cash-Karp stages keep the table path: their
+// item bodies read the arguments so often per site that constant-cache reads
+// cost more than the registers they free (a batch of 16 FP32 RKF45 solves: 9.8
+// against 10.5 G accepted site-updates/s; FP64 Cash-Karp gains 14 %, the RK4
+// stages 4 %).
 template <class S, class C, int K, int TY, bool PAIR, int RR>
-static cudaError_t batch_occupancy(const BatchLaunch& b, int* occupancy) {
+static cudaError_t launch_batch_one(int grid, cudaStream_t st, const BatchLaunch& b, int* occupancy) {
   constexpr bool kParamArgs = !(sizeof(C) == sizeof(float) && K >= K_CK_1 && K <= K_CK_6);
   if constexpr (kParamArgs) {
-    if (b.ns >= 1 && b.ns <= BATCH_PARAM_SOLVES) return batch_setup<S, C, K, TY, PAIR, RR, true>(occupancy);
+    const int rows = grid <= 0 || b.htab ? batch_param_rows(b.ns) : 0;
+    if (rows == BATCH_PARAM_FEW)
+      return grid <= 0 ? batch_setup<S, C, K, TY, PAIR, RR, BATCH_PARAM_FEW>(occupancy)
+                       : launch_batch_rows<S, C, K, TY, PAIR, RR, BATCH_PARAM_FEW>(grid, st, b);
+    if (rows == BATCH_PARAM_SOLVES)
+      return grid <= 0 ? batch_setup<S, C, K, TY, PAIR, RR, BATCH_PARAM_SOLVES>(occupancy)
+                       : launch_batch_rows<S, C, K, TY, PAIR, RR, BATCH_PARAM_SOLVES>(grid, st, b);
   }
-  return batch_setup<S, C, K, TY, PAIR, RR, false>(occupancy);
+  return grid <= 0 ? batch_setup<S, C, K, TY, PAIR, RR, 0>(occupancy)
+                   : launch_batch_rows<S, C, K, TY, PAIR, RR, 0>(grid, st, b);
 }
 
 template <class S, class C, int K, int RR>
 static cudaError_t launch_batch_kind_r(int grid, cudaStream_t st, const BatchLaunch& b, int* occupancy) {
   if constexpr (std::is_same<S, float2>::value && std::is_same<C, float>::value) {
     if constexpr (is_rk4_kind(K)) {
-      if (batch_rk4_f32_rows() == 16) {
-        if (grid <= 0) return batch_occupancy<S, C, K, 16, true, RR>(b, occupancy);
-        return launch_batch_one<S, C, K, 16, true, RR>(grid, st, b);
-      }
+      if (batch_rk4_f32_rows() == 16) return launch_batch_one<S, C, K, 16, true, RR>(grid, st, b, occupancy);
     }
-    if (batch_pair_layout()) {
-      if (grid <= 0) return batch_occupancy<S, C, K, 8, true, RR>(b, occupancy);
-      return launch_batch_one<S, C, K, 8, true, RR>(grid, st, b);
-    }
+    if (batch_pair_layout()) return launch_batch_one<S, C, K, 8, true, RR>(grid, st, b, occupancy);
   }
-  if (grid <= 0) return batch_occupancy<S, C, K, 8, false, RR>(b, occupancy);
-  return launch_batch_one<S, C, K, 8, false, RR>(grid, st, b);
+  return launch_batch_one<S, C, K, 8, false, RR>(grid, st, b, occupancy);
 }
 
 template <class S, class C, int K>

@@ -736,21 +736,26 @@ struct BatchItem {
 };
 
 // The per-solve stage arguments of one batched launch as a kernel parameter
-// (32 KB of parameter space, read through the constant cache): up to
-// BATCH_PARAM_SOLVES solves.  Items index it by their solve, and the item
-// body reads its arguments from there as the single-solve kernels read
-// theirs.  Loaded per item from the global table into registers instead,
-// they keep the kernel at its 128-register bound, and the stages of one
-// 256^3 solve in a pool take 6-8 % longer (a launch with more solves keeps
-// that path).
-constexpr int BATCH_PARAM_SOLVES = 60;
+// (read through the constant cache): up to BATCH_PARAM_SOLVES solves, the 32
+// KB parameter space.  Items index it by their solve, and the item body reads
+// its arguments from there as the single-solve kernels read theirs.  Loaded
+// per item from the global table into registers instead, they keep the kernel
+// at its 128-register bound, and the stages of one 256^3 solve in a pool take
+// 6-8 % longer (a launch with more solves keeps that path).  The parameters
+// travel with every launch (a step of four solves of 24^3: 45 us with 32 KB),
+// so launches of few solves carry BATCH_PARAM_FEW rows (8.4 KB: 35 us).
+constexpr int BATCH_PARAM_SOLVES = 60, BATCH_PARAM_FEW = 16;
+template <int N>
 struct BatchArgs {
-  StageArgs a[BATCH_PARAM_SOLVES];
+  StageArgs a[N];
 };
-struct NoBatchArgs {};
-static_assert(sizeof(BatchArgs) + 256 <= 32764, "batched launch parameters exceed the 32 KB parameter space");
-template <bool PARG>
-using BatchArgsOf = typename std::conditional<PARG, BatchArgs, NoBatchArgs>::type;
+template <>
+struct BatchArgs<0> {};  // the launch reads the device table
+static_assert(sizeof(BatchArgs<BATCH_PARAM_SOLVES>) + 256 <= 32764, "batched launch parameters exceed the 32 KB parameter space");
+// rows the parameters of a launch over ns solves hold, 0 = none
+inline int batch_param_rows(int ns) {
+  return ns < 1 || ns > BATCH_PARAM_SOLVES ? 0 : (ns <= BATCH_PARAM_FEW ? BATCH_PARAM_FEW : BATCH_PARAM_SOLVES);
+}
 
 // One batched launch: tab = the device rows of the ns solves (stage
 // arguments + tensor maps), htab = the same rows on the host.
@@ -792,11 +797,11 @@ __host__ __device__ constexpr int batch_threads() {
 // the stencil radius of every solve the launch serves (a pool keeps solves
 // of the two FD orders in separate classes): one item body per kernel, and
 // rings sized for that radius.
-template <class S, class C, int KIND, int TY, int PY, bool PAIR, int RR, bool PARG>
+template <class S, class C, int KIND, int TY, int PY, bool PAIR, int RR, int PARG>
 __global__ void __launch_bounds__(batch_threads<TY, PY, PAIR>(), (batch_min_blocks<C, KIND, PAIR ? TY : 8>()))
     k_stage_batch(const BatchStage* __restrict__ tab, const BatchItem* __restrict__ items,
                   const int* __restrict__ order, int nitems, int* queue, double* partials,
-                  const __grid_constant__ BatchArgsOf<PARG> pa) {
+                  const __grid_constant__ BatchArgs<PARG> pa) {
   static_assert(!PAIR || (sizeof(S) == 8 && sizeof(C) == 4 && (TY == 8 || TY == 16)),
                 "the pair layout is for complex64 / FP32 on 32 x 8 or 32 x 16 items");
   static_assert(RR == 1 || RR == 2, "stencil radius 1 or 2");
@@ -834,8 +839,8 @@ __global__ void __launch_bounds__(batch_threads<TY, PY, PAIR>(), (batch_min_bloc
                                                     r_err);
     };
     bool ok;
-    if constexpr (PARG) {
-      ok = run(pa.a[it.solve]);  // parameter space: the host puts at most BATCH_PARAM_SOLVES rows there
+    if constexpr (PARG > 0) {
+      ok = run(pa.a[it.solve]);  // parameter space: the host puts at most PARG rows there
     } else {
       // the item's arguments in registers (read-only path, same address for
       // every thread); a shared-memory copy would be re-read after every
