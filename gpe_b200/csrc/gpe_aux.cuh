@@ -207,34 +207,6 @@ static __global__ void __launch_bounds__(256) k_finalize_ranges(const double* __
   }
 }
 
-// Face ghosts of a field whose interior was just written (for example by a
-// strided host-to-device copy).  Rows away from the y and z faces touch their
-// first and last R + 1 sites only.  256^3 complex128: 102 us with a scan of the
-// interior, 43 us so.
-template <class S>
-__global__ void __launch_bounds__(ROW_THREADS) k_fill_ghosts(S* f, Geom g, int R, int bcs) {
-  for_each_row(g, [&](int k, int j, int lane, long long) {
-    S* row = f + (long long)(k + 2) * g.pz + (long long)(j + 2) * g.px + g.xoff;
-    const int gy = ghost_pos(j, g.ny, R, bcs), gz = ghost_pos(k, g.nz, R, bcs);
-    if (gy == NOGHOST && gz == NOGHOST) {
-      // sites 0 .. R and nx-1-R .. nx-1 (nx >= 6 keeps the two ends apart)
-      const int i = lane <= R ? lane : g.nx - 2 - 2 * R + lane;
-      if (lane < 2 * R + 2 && i < g.nx) {
-        const int gx = ghost_pos(i, g.nx, R, bcs);
-        if (gx != NOGHOST) row[gx] = row[i];
-      }
-      return;
-    }
-    for (int i = lane; i < g.nx; i += 32) {
-      const S v = row[i];
-      const int gx = ghost_pos(i, g.nx, R, bcs);
-      if (gx != NOGHOST) row[gx] = v;
-      if (gy != NOGHOST) row[(long long)(gy - j) * g.px + i] = v;
-      if (gz != NOGHOST) row[(long long)(gz - k) * g.pz + i] = v;
-    }
-  });
-}
-
 // renormalise (variables.f90:715-726): var = sqrt(nn)*var/sqrt(norm), over
 // the whole padded buffer (ghost copies scale identically)
 template <class S>

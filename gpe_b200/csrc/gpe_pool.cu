@@ -117,6 +117,7 @@ struct Solve {
   void* out = nullptr;
   int status = GPE_OK;
   double t_submit = 0, t_start = -1;
+  size_t interior_bytes() const { return (size_t)g.nx * g.ny * g.nz * esz; }
   CUtensorMap halo[9], pw[9];
 };
 
@@ -267,36 +268,32 @@ int grid_for(int cls, int kind, int nitems, int ns) {
   return std::max(1, std::min(nitems, occ));
 }
 
-// Copy a contiguous host interior into field f of a solve, then its ghosts.
-int upload_state(gpe_pool* P, Solve* s, const void* psi, int fidx) {
-  cudaMemcpy3DParms m;
-  memset(&m, 0, sizeof(m));
-  m.srcPtr = make_cudaPitchedPtr(const_cast<void*>(psi), (size_t)s->g.nx * s->esz, (size_t)s->g.nx * s->esz,
-                                 (size_t)s->g.ny);
-  m.dstPtr = make_cudaPitchedPtr(s->f[fidx], (size_t)s->g.px * s->esz, (size_t)s->g.px * s->esz,
-                                 (size_t)(s->g.ny + 4));
-  m.dstPos = make_cudaPos((size_t)s->g.xoff * s->esz, 2, 2);
-  m.extent = make_cudaExtent((size_t)s->g.nx * s->esz, (size_t)s->g.ny, (size_t)s->g.nz);
-  m.kind = cudaMemcpyHostToDevice;
-  PCU(P, cudaMemcpy3DAsync(&m, P->st));
+// A solve's state crosses the bus as one contiguous block, through a field
+// that is free at the time, and is packed (with its ghosts) or unpacked on the
+// device: a strided copy moves rows of nx elements, and a few hundred bytes a
+// row is far from the bus's rate (16 solves of 32^3-128^3: 5.5 ms for the
+// uploads with it, 1.9 so).
+int upload_state(gpe_pool* P, Solve* s, const void* psi) {
+  void* stage = s->f[1];  // free until the first step
+  PCU(P, cudaMemcpyAsync(stage, psi, s->interior_bytes(), cudaMemcpyHostToDevice, P->st));
   if (s->esz == 16)
-    k_fill_ghosts<double2><<<ROW_GRID, ROW_THREADS, 0, P->st>>>((double2*)s->f[fidx], s->g, s->R, s->p.bcs);
+    k_pack<double2, double2><<<ROW_GRID, ROW_THREADS, 0, P->st>>>((const double2*)stage, (double2*)s->f[0], s->g, s->R,
+                                                                  s->p.bcs);
   else
-    k_fill_ghosts<float2><<<ROW_GRID, ROW_THREADS, 0, P->st>>>((float2*)s->f[fidx], s->g, s->R, s->p.bcs);
+    k_pack<float2, float2><<<ROW_GRID, ROW_THREADS, 0, P->st>>>((const float2*)stage, (float2*)s->f[0], s->g, s->R,
+                                                                s->p.bcs);
   PCU(P, cudaGetLastError());
   return GPE_OK;
 }
 
 int download_state(gpe_pool* P, Solve* s, int fidx) {
-  cudaMemcpy3DParms m;
-  memset(&m, 0, sizeof(m));
-  m.srcPtr = make_cudaPitchedPtr(s->f[fidx], (size_t)s->g.px * s->esz, (size_t)s->g.px * s->esz,
-                                 (size_t)(s->g.ny + 4));
-  m.srcPos = make_cudaPos((size_t)s->g.xoff * s->esz, 2, 2);
-  m.dstPtr = make_cudaPitchedPtr(s->out, (size_t)s->g.nx * s->esz, (size_t)s->g.nx * s->esz, (size_t)s->g.ny);
-  m.extent = make_cudaExtent((size_t)s->g.nx * s->esz, (size_t)s->g.ny, (size_t)s->g.nz);
-  m.kind = cudaMemcpyDeviceToHost;
-  PCU(P, cudaMemcpy3DAsync(&m, P->st));
+  void* stage = s->f[2];  // a stage field: the solve is done stepping
+  if (s->esz == 16)
+    k_unpack<double2, double2><<<ROW_GRID, ROW_THREADS, 0, P->st>>>((const double2*)s->f[fidx], (double2*)stage, s->g);
+  else
+    k_unpack<float2, float2><<<ROW_GRID, ROW_THREADS, 0, P->st>>>((const float2*)s->f[fidx], (float2*)stage, s->g);
+  PCU(P, cudaGetLastError());
+  PCU(P, cudaMemcpyAsync(s->out, stage, s->interior_bytes(), cudaMemcpyDeviceToHost, P->st));
   return GPE_OK;
 }
 
@@ -760,7 +757,7 @@ static int pool_submit_impl(gpe_pool* P, const gpe_params* prm, const void* psi0
           cudaSuccess)
     return bail(GPE_ERR_CUDA, "upload of tables failed");
   if (psi0) {
-    if (int rc = upload_state(P, s, psi0, 0)) return bail(rc, P->err);
+    if (int rc = upload_state(P, s, psi0)) return bail(rc, P->err);
   } else {
     // the other fields are free until the first step: the generator's
     // scratch (spectrum + FFT) lives there

@@ -35,7 +35,7 @@ def test_pack_ghosts_unpack(gpu, nx, storage, bcs, order):
     ref = Oracle(rp.replace(storage="c128", compute="auto")).energy(held)
     scale = np.sum(np.abs(held) ** 2) * 400.0 * 0.125
     assert abs(e - ref) <= scale * (1e-13 if storage == "c128" else 1e-6)
-    # the pool fills its ghosts from the copied interior: one step equals the handle's, bitwise
+    # the pool packs its copy of the interior: one step equals the handle's, bitwise
     pool = Pool(Pool.solve_bytes(rp) + (32 << 20))
     assert pool.submit(rp, held.astype(ct), 1, 0)
     (r,) = pool.run_all()
