@@ -146,8 +146,11 @@ __global__ void __launch_bounds__(ROW_THREADS) k_norm_batch(const NormSolve* __r
   block_reduce_store_at<ROW_THREADS>(s, 0.0, 0.0, partials, blockIdx.x);
 }
 
-// Sum (slots 0,1) and max (slot 2) of nb block partials in a fixed order.
-static __global__ void __launch_bounds__(256) k_finalize(const double* __restrict__ partials, long long nb, double* out) {
+// Sum (slots 0,1) and max (slot 2) of nb block partials in a fixed order;
+// zeroes *top (the running maximum of the stage that made them) for its next
+// launch.
+static __global__ void __launch_bounds__(256) k_finalize(const double* __restrict__ partials, long long nb, double* out,
+                                                         unsigned long long* top) {
   __shared__ double s0[256], s1[256], s2[256];
   const int t = threadIdx.x;
   double a = 0.0, b = 0.0, c = 0.0;
@@ -172,6 +175,7 @@ static __global__ void __launch_bounds__(256) k_finalize(const double* __restric
     out[0] = s0[0];
     out[1] = s1[0];
     out[2] = s2[0];
+    *top = 0;
   }
 }
 

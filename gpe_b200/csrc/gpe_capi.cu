@@ -72,7 +72,7 @@ struct gpe_handle {
   long long part_cap = 0;    // blocks it holds
   dim3 norm_grid;            // k_norm's grid: 32 x 8 tiles x z-chunks of zc planes
   long long norm_npart = 0;  // its partials
-  double* dres = nullptr;    // [6] finalised reductions, then the status word
+  double* dres = nullptr;    // [6] finalised reductions, the status word, err_top
   double* hres = nullptr;    // pinned mirror of dres and the status word
   void* staging = nullptr;
   size_t staging_bytes = 0;
@@ -391,8 +391,12 @@ StageArgs base_args(gpe_handle* h) {
   return a;
 }
 
+// the running error maximum of Cash-Karp stage 6 (StageArgs::kout), behind the
+// results; every finalisation leaves it zero
+unsigned long long* err_top(gpe_handle* h) { return (unsigned long long*)(h->dres + 7); }
+
 int finalize_into(gpe_handle* h, int slot, long long nparts) {
-  k_finalize<<<1, 256, 0, h->st>>>(h->part, nparts, h->dres + 3 * slot);
+  k_finalize<<<1, 256, 0, h->st>>>(h->part, nparts, h->dres + 3 * slot, err_top(h));
   CU(h, cudaGetLastError());
   return GPE_OK;
 }
@@ -563,7 +567,7 @@ int rk45_step(gpe_handle* h, gpe_step_info* io, bool energy, bool norm) {
       a.in = ins[m];
       a.out = outs[m];
       for (int q = 0; q < 5; ++q) a.b[q] = 0.0;
-      a.kout = m < 5 ? K[m] : nullptr;
+      a.kout = m < 5 ? K[m] : (void*)err_top(h);
       if (m < 5) {
         for (int q = 0; q <= m; ++q) a.b[q] = CK_B[m][q];
         for (int q = 0; q < m; ++q) a.kin[q] = K[q];
@@ -818,13 +822,13 @@ int create_impl(const gpe_params* p, const SlabSpec* sp, gpe_handle** out) {
   std::vector<double> tab;
   build_tables(h, tab);
   if (cudaMalloc(&h->tables, tab.size() * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&h->dres, RESULT_BYTES) != cudaSuccess || cudaMallocHost(&h->hres, RESULT_BYTES) != cudaSuccess) {
+      cudaMalloc(&h->dres, RESULT_BYTES + sizeof(unsigned long long)) != cudaSuccess || cudaMallocHost(&h->hres, RESULT_BYTES) != cudaSuccess) {
     cudaGetLastError();
     h->err = "out of memory allocating tables / reduction buffers";
     return bail(GPE_ERR_NOMEM);
   }
   cudaMemcpyAsync(h->tables, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, h->st);
-  cudaMemsetAsync(h->dres, 0, RESULT_BYTES, h->st);
+  cudaMemsetAsync(h->dres, 0, RESULT_BYTES + sizeof(unsigned long long), h->st);
   h->status = (int*)(h->dres + 6);
   if (cudaStreamSynchronize(h->st) != cudaSuccess) {
     h->err = "initialisation failed";
