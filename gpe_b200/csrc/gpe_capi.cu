@@ -1029,6 +1029,10 @@ static int ensure_step_graph(gpe_handle* h, int which, double dr, double di) {
   return GPE_OK;
 }
 
+static bool have_step_graph(const gpe_handle* h, double dr, double di) {
+  return h->graph_dr == dr && h->graph_di == di && (h->step_graph[0] || h->step_graph[1]);
+}
+
 static bool use_step_graphs(const gpe_handle* h) {
   static const bool off = [] {
     const char* e = getenv("GPE_GRAPHS");
@@ -1054,16 +1058,15 @@ static int step_impl(gpe_handle* h, int64_t nsteps, gpe_step_info* io, bool wait
   } else {
     const double dr = io->dt_re, di = io->dt_im;
     // steps without reductions replay a captured graph (one launch instead of
-    // one per stage); the first step of a call runs plainly, so every kernel
-    // has been loaded and configured before any capture
-    // (a step with a norm from its second use on: a relaxation asks for one
-    // per call)
+    // one per stage); before any capture a step runs plainly, so that every
+    // kernel has been loaded and configured (a step with a norm: from its
+    // second use on, as a relaxation asks for one per call)
     const bool can = use_step_graphs(h), graphs = can && nsteps >= 3;
     bool copied = false;
     for (int64_t s = 0; s < nsteps;) {
       const bool e = want_e && s == 0, n = want_n && s == nsteps - 1;
       int64_t took = 1;
-      if (graphs && s > 0 && !e && !n) {
+      if (graphs && (s > 0 || have_step_graph(h, dr, di)) && !e && !n) {
         const int64_t left = nsteps - s - (want_n ? 1 : 0);  // steps without reductions
         const int which = left >= GRAPH_STEPS ? 1 : 0;
         if (int rc = ensure_step_graph(h, which, dr, di)) return rc;
