@@ -121,8 +121,10 @@ struct gpe_handle {
   // graph launch and its gap once per GRAPH_STEPS steps; [2] one step with
   // the norm of its result and the copy of the results to the host
   cudaGraphExec_t step_graph[3] = {nullptr, nullptr, nullptr};
-  int64_t norm_steps = 0;  // steps with a norm so far (the second one captures)
-  double graph_dr = 0, graph_di = 0;
+  double graph_dt[3][2] = {};  // the dt of each
+  // dt of the last call and of the last step with a norm: what a graph costs
+  // to capture pays from the second use of a dt on
+  double call_dt[2] = {}, norm_dt[2] = {};
   bool capturing = false;  // stage launches become dependents of each other
   // asynchronous state copies (gpe_set_state_async / gpe_get_state_async):
   // host <-> staging transfers on a copy stream, pack/unpack on the solve's
@@ -998,16 +1000,24 @@ int gpe_get_state_device(gpe_handle* h, void* psi_dev, int32_t dtype) {
 // or of one with the norm and the results' copy (2), captured on first use and
 // whenever dt changes.  Only for schemes that keep psi in place.
 constexpr int GRAPH_STEPS = 8;
+static bool have_step_graph(const gpe_handle* h, int which, double dr, double di) {
+  return h->step_graph[which] && h->graph_dt[which][0] == dr && h->graph_dt[which][1] == di;
+}
+
+// Is (dr, di) the dt kept in last?  Keeps it.
+static bool same_dt(double (&last)[2], double dr, double di) {
+  const bool same = last[0] == dr && last[1] == di;
+  last[0] = dr;
+  last[1] = di;
+  return same;
+}
+
 static int ensure_step_graph(gpe_handle* h, int which, double dr, double di) {
-  if (h->graph_dr != dr || h->graph_di != di) {
-    for (cudaGraphExec_t& g : h->step_graph) {
-      if (g) cudaGraphExecDestroy(g);
-      g = nullptr;
-    }
-    h->graph_dr = dr;
-    h->graph_di = di;
-  }
-  if (h->step_graph[which]) return GPE_OK;
+  if (have_step_graph(h, which, dr, di)) return GPE_OK;
+  if (h->step_graph[which]) cudaGraphExecDestroy(h->step_graph[which]);
+  h->step_graph[which] = nullptr;
+  h->graph_dt[which][0] = dr;
+  h->graph_dt[which][1] = di;
   cudaGraph_t g = nullptr;
   CU(h, cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
   h->capturing = true;
@@ -1027,10 +1037,6 @@ static int ensure_step_graph(gpe_handle* h, int which, double dr, double di) {
   if (ei != cudaSuccess) h->step_graph[which] = nullptr;
   CU(h, ei);
   return GPE_OK;
-}
-
-static bool have_step_graph(const gpe_handle* h, double dr, double di) {
-  return h->graph_dr == dr && h->graph_di == di && (h->step_graph[0] || h->step_graph[1]);
 }
 
 static bool use_step_graphs(const gpe_handle* h) {
@@ -1059,20 +1065,24 @@ static int step_impl(gpe_handle* h, int64_t nsteps, gpe_step_info* io, bool wait
     const double dr = io->dt_re, di = io->dt_im;
     // steps without reductions replay a captured graph (one launch instead of
     // one per stage); before any capture a step runs plainly, so that every
-    // kernel has been loaded and configured (a step with a norm: from its
-    // second use on, as a relaxation asks for one per call)
+    // kernel has been loaded and configured.  The graph of GRAPH_STEPS steps is
+    // captured for long calls, else when a dt comes again; that of a step with
+    // a norm when the last one had the same dt (a relaxation asks for one per
+    // call)
     const bool can = use_step_graphs(h), graphs = can && nsteps >= 3;
+    const bool again = same_dt(h->call_dt, dr, di);
+    const bool have = have_step_graph(h, 0, dr, di) || have_step_graph(h, 1, dr, di);
     bool copied = false;
     for (int64_t s = 0; s < nsteps;) {
       const bool e = want_e && s == 0, n = want_n && s == nsteps - 1;
       int64_t took = 1;
-      if (graphs && (s > 0 || have_step_graph(h, dr, di)) && !e && !n) {
+      if (graphs && (s > 0 || have) && !e && !n) {
         const int64_t left = nsteps - s - (want_n ? 1 : 0);  // steps without reductions
-        const int which = left >= GRAPH_STEPS ? 1 : 0;
+        const int which = left >= GRAPH_STEPS && (again || left >= 4 * GRAPH_STEPS || have_step_graph(h, 1, dr, di));
         if (int rc = ensure_step_graph(h, which, dr, di)) return rc;
         CU(h, cudaGraphLaunch(h->step_graph[which], h->st));
         if (which) took = GRAPH_STEPS;
-      } else if (can && n && !e && h->norm_steps++ > 0) {
+      } else if (can && n && !e && same_dt(h->norm_dt, dr, di)) {
         if (int rc = ensure_step_graph(h, 2, dr, di)) return rc;
         CU(h, cudaGraphLaunch(h->step_graph[2], h->st));
         copied = true;

@@ -34,3 +34,26 @@ def test_many_steps_equal_single_calls(gpu, shape, storage, scheme):
             assert a.norm == b.norm
     one.close()
     many.close()
+
+
+def test_changing_time_steps(gpu):
+    # graphs belong to a dt: each comes back, changes after one call, and
+    # alternates from call to call, with and without a norm
+    rp = RunParams(nx=20, ny=18, nz=16, xr=4.75, yr=4.25, zr=3.75, tau=0.004, scheme="rk4", eqn_to_solve=2, bcs=1, order=4)
+    rng = np.random.default_rng(7)
+    psi0 = 1.0 + 0.1 * (rng.normal(size=(16, 18, 20)) + 1j * rng.normal(size=(16, 18, 20)))
+    one, many = Solver(rp), Solver(rp)
+    one.set_state(psi0)
+    many.set_state(psi0)
+    for n, dt, norm in [(10, 4e-3, True), (10, 4e-3, True), (10, 2e-3, True), (1, 4e-3, True), (1, 4e-3, True),
+                        (1, 2e-3, True), (1, 4e-3, True), (40, 2e-3, False), (9, 4e-3, False), (9, 2e-3, True)]:
+        one.dt = many.dt = complex(dt, 0.0)
+        for _ in range(n):
+            one.solver(1)
+        b = many.solver(n, want_norm=norm)
+        np.testing.assert_array_equal(many.get_state(), one.get_state(), err_msg=f"{n} steps of {dt}")
+        assert one.t == many.t
+        if norm:
+            assert b.norm == pytest.approx(one.get_norm(), rel=16 * 18 * 20 * 2.3e-16)
+    one.close()
+    many.close()
