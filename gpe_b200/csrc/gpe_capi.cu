@@ -188,10 +188,10 @@ int chunk_of(gpe_handle* h, int kind) {
   const int th = tile_rows(h->tma_ty);
   const long long tiles = (long long)((h->p.nx + 31) / 32) * ((h->p.ny + th - 1) / th);
   int per = 0;
-  if (h->p.tile_zc > 0) {
+  if (h->tma_ty == TILE_SITE) {
+    zc = 1;  // its blocks have no z loop: a chunk asked for would leave planes out
+  } else if (h->p.tile_zc > 0) {
     zc = std::min(h->p.tile_zc, h->p.nz);
-  } else if (h->tma_ty == TILE_SITE) {
-    zc = 1;
   } else if (!h->use_tma) {
     zc = default_zc(h->g, th, h->esz);
   } else {
