@@ -77,6 +77,7 @@ struct gpe_handle {
   void* staging = nullptr;
   size_t staging_bytes = 0;
   int zc = 8;                // planes per block of k_norm
+  int zc_asked = 0;          // planes per CTA asked for at creation (tile_zc, else GPE_ZC), 0 = none
   int zck[K_NUM] = {0};      // planes per CTA of each stage kernel launched so far (chunk_of)
   int nsm = 148;             // SMs of the device
   std::string err;
@@ -190,8 +191,8 @@ int chunk_of(gpe_handle* h, int kind) {
   int per = 0;
   if (h->tma_ty == TILE_SITE) {
     zc = 1;  // its blocks have no z loop: a chunk asked for would leave planes out
-  } else if (h->p.tile_zc > 0) {
-    zc = std::min(h->p.tile_zc, h->p.nz);
+  } else if (h->zc_asked) {
+    zc = h->zc_asked;
   } else if (!h->use_tma) {
     zc = default_zc(h->g, th, h->esz);
   } else {
@@ -771,6 +772,7 @@ int create_impl(const gpe_params* p, const SlabSpec* sp, gpe_handle** out) {
   h->R = p->order / 2;
   h->cmode = p->storage == GPE_C128 ? CM_F64 : (p->compute == GPE_COMPUTE_F64 ? CM_F32X : CM_F32);
   h->nelem = padded_elems(h->g);
+  h->zc_asked = p->tile_zc > 0 ? std::min(p->tile_zc, pl.nz) : zc_from_env(pl.nz);
   // thread layout: complex64 storage with the FP32 stencil takes two
   // x-adjacent sites per thread (16-byte shared-memory reads and stores)
   if (const char* e = getenv("GPE_KERNEL")) h->use_tma = strcmp(e, "ldg") != 0;
@@ -781,12 +783,12 @@ int create_impl(const gpe_params* p, const SlabSpec* sp, gpe_handle** out) {
     if (v == TILE_32x8_ROW1 || v == TILE_32x8_ROW2 || v == TILE_SITE ||
         (h->cmode == CM_F32 && h->use_tma && tile_is_pair(v)))
       h->tma_ty = v;
-  } else if (h->use_tma && p->tile_zc == 0 && !getenv("GPE_ROWS_PER_THREAD") && !getenv("GPE_ZC") &&
+  } else if (h->use_tma && !h->zc_asked && !getenv("GPE_ROWS_PER_THREAD") &&
              (long long)((pl.nx + 31) / 32) * ((pl.ny + SITE_TY - 1) / SITE_TY) * pl.nz <= SITE_MAX_BLOCKS) {
     h->tma_ty = TILE_SITE;  // a small grid, and no layout or chunk asked for
   }
   h->nsm = prop.multiProcessorCount;
-  h->zc = p->tile_zc > 0 ? std::min(p->tile_zc, pl.nz) : default_zc(h->g, tile_rows(h->tma_ty), h->esz);
+  h->zc = h->zc_asked ? h->zc_asked : default_zc(h->g, tile_rows(h->tma_ty), h->esz);
   h->norm_grid = dim3((pl.nx + 31) / 32, (pl.ny + 7) / 8, (pl.nz + h->zc - 1) / h->zc);
   h->norm_npart = (long long)h->norm_grid.x * h->norm_grid.y * h->norm_grid.z;
   auto bail = [&](int rc) {

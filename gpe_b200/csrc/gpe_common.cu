@@ -57,7 +57,7 @@ int scheme_fields(int scheme) {
 }
 
 // GPE_ZC: planes per CTA asked for by name, 0 = none
-static int zc_from_env(int nz) {
+int zc_from_env(int nz) {
   const char* e = getenv("GPE_ZC");
   const int v = e ? atoi(e) : 0;
   return v > 0 ? std::min(v, nz) : 0;
@@ -77,7 +77,6 @@ static int zc_from_env(int nz) {
 // storages, the choice is within 0.6 % of the best chunk on average (7 % at
 // worst) and 15 % faster than a fixed target of 8 CTAs per SM.
 int balanced_zc(const Geom& g, int esz, int R, long long tiles, long long slots) {
-  if (const int v = zc_from_env(g.nz)) return v;
   const double lead = 5 * R - 4;
   const int zmax = std::min(g.nz, esz >= 16 ? 24 : 20);
   int best = 1;
@@ -97,7 +96,6 @@ int balanced_zc(const Geom& g, int esz, int R, long long tiles, long long slots)
 // z planes per block: enough blocks for several waves on 148 SMs (the norm
 // kernel and k_stage)
 int default_zc(const Geom& g, int tile_h, int esz) {
-  if (const int v = zc_from_env(g.nz)) return v;
   const long long bxy = (long long)((g.nx + 31) / 32) * ((g.ny + tile_h - 1) / tile_h);
   const long long target = 148LL * 8;
   const long long cap = esz >= 16 ? 24 : 20;

@@ -22,6 +22,8 @@ void param_layout(const gpe_params* p, Geom& g, int& esz);
 long long padded_elems(const Geom& g);
 // fields a scheme keeps per solve
 int scheme_fields(int scheme);
+// z planes per CTA asked for in the environment (GPE_ZC), 0 = none
+int zc_from_env(int nz);
 // z planes per CTA of a stage launch over `tiles` x-y tiles when `slots` CTAs
 // of the kernel run at once on the device
 int balanced_zc(const Geom& g, int esz, int R, long long tiles, long long slots);

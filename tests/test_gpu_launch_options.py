@@ -42,3 +42,23 @@ def test_a_thread_per_site_updates_every_plane(gpu, monkeypatch, zc, scheme):
         s.close()
     np.testing.assert_array_equal(out[1][0], out[0][0])
     assert out[1][1:] == out[0][1:]
+
+
+# the partition of a launch fixes the order of its sums, so equal norms of
+# eight states say that both handles cut their launches alike
+@pytest.mark.parametrize("storage", ["c128", "c64"])
+def test_the_environment_counts_when_a_handle_is_created(gpu, monkeypatch, storage):
+    shape = (96, 96, 96)
+    norms = []
+    for keep in (True, False):
+        monkeypatch.setenv("GPE_ZC", "17")
+        s = Solver(params(shape, storage=storage))
+        if not keep:
+            monkeypatch.delenv("GPE_ZC")
+        row = []
+        for seed in range(8):
+            s.set_state(noise(shape, seed))
+            row.append(s.solver(1, want_norm=True).norm)
+        norms.append(row)
+        s.close()
+    assert norms[0] == norms[1]
