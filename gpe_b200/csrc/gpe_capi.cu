@@ -68,7 +68,10 @@ struct gpe_handle {
   double* tables = nullptr;
   std::vector<double> x, y, z;
   double dx = 0, dy = 0, dz = 0;
-  double* part = nullptr;    // block partials of a reduction, finalised before the next one
+  // block partials of a reduction, finalised before the next one.  Made at
+  // creation for the largest launch there can be: captured steps hold its
+  // address, so it lives as long as the handle
+  double* part = nullptr;
   long long part_cap = 0;    // blocks it holds
   dim3 norm_grid;            // k_norm's grid: 32 x 8 tiles x z-chunks of zc planes
   long long norm_npart = 0;  // its partials
@@ -180,36 +183,44 @@ int field_of(const gpe_handle* h, const void* p) {
   return -1;
 }
 
+// Planes per CTA that do not depend on the kernel's CTAs per SM, 0 = they do.
+int fixed_chunk(const gpe_handle* h) {
+  if (h->tma_ty == TILE_SITE) return 1;  // its blocks have no z loop: a chunk asked for would leave planes out
+  if (h->zc_asked) return h->zc_asked;
+  return h->use_tma ? 0 : default_zc(h->g, tile_rows(h->tma_ty), h->esz);
+}
+
+// grid of a stage launch: x-y tiles times z-chunks of zc planes
+dim3 chunk_grid(const gpe_handle* h, int zc) {
+  const int th = tile_rows(h->tma_ty);
+  return dim3((h->p.nx + 31) / 32, (h->p.ny + th - 1) / th, (h->p.nz + zc - 1) / zc);
+}
+
+// Planes per CTA of a stage kernel of which `per` CTAs fit on an SM.
+int chunk_for(const gpe_handle* h, int per) {
+  const dim3 g = chunk_grid(h, h->p.nz);
+  return balanced_zc(h->g, h->esz, h->R, (long long)g.x * g.y, (long long)h->nsm * per);
+}
+
 // Planes per CTA of a stage kernel, chosen at its first launch by the kernel's
 // CTAs per SM (the Cash-Karp stages with many point-wise inputs hold half as
 // many as the others).
+constexpr int STAGE_MAX_CTAS = 16;  // per SM: 2048 threads in CTAs of 128, the smallest a march has
 int chunk_of(gpe_handle* h, int kind) {
   int& zc = h->zck[kind];
-  if (zc) return zc;
-  const int th = tile_rows(h->tma_ty);
-  const long long tiles = (long long)((h->p.nx + 31) / 32) * ((h->p.ny + th - 1) / th);
-  int per = 0;
-  if (h->tma_ty == TILE_SITE) {
-    zc = 1;  // its blocks have no z loop: a chunk asked for would leave planes out
-  } else if (h->zc_asked) {
-    zc = h->zc_asked;
-  } else if (!h->use_tma) {
-    zc = default_zc(h->g, th, h->esz);
-  } else {
+  if (!zc) zc = fixed_chunk(h);
+  if (!zc) {
+    int per = 0;
     const cudaError_t e = h->cmode == CM_F64   ? stage_tma_occupancy_f64(kind, h->R, h->tma_ty, &per)
                           : h->cmode == CM_F32 ? stage_tma_occupancy_f32(kind, h->R, h->tma_ty, &per)
                                                : stage_tma_occupancy_f32x(kind, h->R, h->tma_ty, &per);
     // (a kernel that cannot be queried cannot be launched either)
-    zc = balanced_zc(h->g, h->esz, h->R, tiles, (long long)h->nsm * (e == cudaSuccess && per > 0 ? per : 1));
+    zc = chunk_for(h, e == cudaSuccess && per > 0 ? std::min(per, STAGE_MAX_CTAS) : 1);
   }
   return zc;
 }
 
-// grid of a stage launch: x-y tiles times z-chunks of the kind's length
-dim3 stage_grid(gpe_handle* h, int kind) {
-  const int th = tile_rows(h->tma_ty), zc = chunk_of(h, kind);
-  return dim3((h->p.nx + 31) / 32, (h->p.ny + th - 1) / th, (h->p.nz + zc - 1) / zc);
-}
+dim3 stage_grid(gpe_handle* h, int kind) { return chunk_grid(h, chunk_of(h, kind)); }
 
 // partials of a stage launch, one per CTA
 long long stage_parts(gpe_handle* h, int kind) {
@@ -217,21 +228,17 @@ long long stage_parts(gpe_handle* h, int kind) {
   return (long long)g.x * g.y * g.z;
 }
 
-// Make room for the partials of n blocks.
-int ensure_parts(gpe_handle* h, long long n) {
-  if (n <= h->part_cap) return GPE_OK;
-  if (h->part) {
-    CU(h, cudaStreamSynchronize(h->st));
-    cudaFree(h->part);
-    h->part = nullptr;
-    h->part_cap = 0;
+// The most partials a reduction of the handle can have: those of k_norm, and
+// of the stage kernels whatever CTAs per SM they turn out to have (asking for
+// them would load every kernel at creation).
+long long most_parts(const gpe_handle* h) {
+  int zc = fixed_chunk(h);
+  if (!zc) {
+    zc = h->p.nz;
+    for (int per = 1; per <= STAGE_MAX_CTAS; ++per) zc = std::min(zc, chunk_for(h, per));
   }
-  if (cudaMalloc(&h->part, n * RED_SLOTS * sizeof(double)) != cudaSuccess) {
-    cudaGetLastError();
-    return fail(h, GPE_ERR_NOMEM, "out of device memory for the partials of a reduction");
-  }
-  h->part_cap = n;
-  return GPE_OK;
+  const dim3 g = chunk_grid(h, zc);
+  return std::max((long long)g.x * g.y * g.z, h->norm_npart);
 }
 
 cudaError_t launch_raw(gpe_handle* h, int kind, const StageArgs& a_in) {
@@ -239,6 +246,7 @@ cudaError_t launch_raw(gpe_handle* h, int kind, const StageArgs& a_in) {
   a.status = h->status;
   a.zc = chunk_of(h, kind);
   const dim3 grid = stage_grid(h, kind);
+  if (a.partials && stage_parts(h, kind) > h->part_cap) return cudaErrorInvalidValue;  // (most_parts rules it out)
   set_f32_constants(a);
   if (!h->use_tma || h->tma_ty == TILE_SITE) {
     const int ty = h->tma_ty == TILE_SITE ? TILE_SITE : 8;
@@ -469,12 +477,6 @@ int enqueue_fixed_step(gpe_handle* h, double dr, double di, bool energy, bool no
   StageArgs a = base_args(h);
   void** F = h->fields.data();
   const int sc = h->p.scheme;
-  if (energy || norm) {
-    const int first = sc == GPE_RK4 ? K_RK4_1 : (sc == GPE_RK2 ? K_RK2_1 : K_EULER);
-    const int last = sc == GPE_RK4 ? K_RK4_4 : (sc == GPE_RK2 ? K_RK2_2 : K_EULER);
-    if (int rc = ensure_parts(h, std::max(energy ? stage_parts(h, first) : 0, norm ? stage_parts(h, last) : 0)))
-      return rc;
-  }
   if (sc == GPE_RK4) {
     void *psi = F[0], *A = F[1], *B = F[2], *Q = F[3];
     // s1: k1 = f(psi); A = psi + dt/2 k1
@@ -557,7 +559,6 @@ int rk45_step(gpe_handle* h, gpe_step_info* io, bool energy, bool norm) {
   void* K[5] = {F[4], F[5], F[6], F[7], F[8]};
   double errmax = 0.0;
   bool first = true;
-  if (int rc = ensure_parts(h, std::max(stage_parts(h, K_CK_6), energy ? stage_parts(h, K_CK_1) : 0))) return rc;
   for (int attempt = 0;; ++attempt) {
     if (attempt > 10000) return fail(h, GPE_ERR_STATE, "rkqs: no acceptable step after 10000 attempts");
     StageArgs a = base_args(h);
@@ -624,7 +625,6 @@ int norm_now(gpe_handle* h, double* out) {
   const Geom& g = h->g;
   const size_t ntot = (size_t)h->p.nx + h->p.ny + h->p.nz;
   const double* w = h->tables + 2 * ntot;
-  if (int rc = ensure_parts(h, h->norm_npart)) return rc;
   if (h->esz == 16)
     k_norm<double2><<<h->norm_grid, dim3(32, 8), 0, h->st>>>((const double2*)h->fields[h->cur], g, h->zc, w,
                                                              w + g.nx, w + g.nx + g.ny, h->part);
@@ -825,8 +825,11 @@ int create_impl(const gpe_params* p, const SlabSpec* sp, gpe_handle** out) {
   }
   std::vector<double> tab;
   build_tables(h, tab);
+  h->part_cap = most_parts(h);
   if (cudaMalloc(&h->tables, tab.size() * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&h->dres, RESULT_BYTES + sizeof(unsigned long long)) != cudaSuccess || cudaMallocHost(&h->hres, RESULT_BYTES) != cudaSuccess) {
+      cudaMalloc(&h->part, h->part_cap * RED_SLOTS * sizeof(double)) != cudaSuccess ||
+      cudaMalloc(&h->dres, RESULT_BYTES + sizeof(unsigned long long)) != cudaSuccess ||
+      cudaMallocHost(&h->hres, RESULT_BYTES) != cudaSuccess) {
     cudaGetLastError();
     h->err = "out of memory allocating tables / reduction buffers";
     return bail(GPE_ERR_NOMEM);
@@ -1241,7 +1244,6 @@ int gpe_energy(gpe_handle* h, double* energy) {
   StageArgs a = base_args(h);
   a.in = h->fields[h->cur];
   a.want_energy = 1;
-  if (int rc = ensure_parts(h, stage_parts(h, K_ENERGY))) return rc;
   a.partials = h->part;
   CU(h, launch(h, K_ENERGY, a));
   if (int rc = finalize_into(h, 0, stage_parts(h, K_ENERGY))) return rc;

@@ -57,3 +57,45 @@ def test_changing_time_steps(gpu):
             assert b.norm == pytest.approx(one.get_norm(), rel=16 * 18 * 20 * 2.3e-16)
     one.close()
     many.close()
+
+
+# (the shapes march, and their norm and energy launches have more blocks than
+# the last stage; complex64 has the layout of two sites a thread)
+@pytest.mark.parametrize("n,storage", [(96, "c128"), (128, "c64")])
+@pytest.mark.parametrize("scheme", ["rk4", "rk2"])
+def test_other_reductions_between_steps_with_a_norm(gpu, n, storage, scheme):
+    # a captured step with a norm keeps the address of its block partials:
+    # other reductions of the handle, and a second handle's memory, leave it
+    # as it is
+    h = 0.25 * (n - 1)
+    rp = RunParams(nx=n, ny=n, nz=n, xr=h, yr=h, zr=h, tau=0.004, scheme=scheme, eqn_to_solve=2, bcs=1, order=4,
+                   storage=storage)
+    rng = np.random.default_rng(n)
+    psi0 = 1.0 + 0.1 * (rng.normal(size=(n, n, n)) + 1j * rng.normal(size=(n, n, n)))
+    with Solver(rp) as s:  # alone: plain steps, no reduction before the last
+        s.set_state(psi0)
+        for _ in range(5):
+            s.solver(1)
+        alone, norm_alone = s.get_state(), s.get_norm()
+        s.set_state(psi0)
+        s.solver(1)
+        second_alone = s.get_state()
+    first = Solver(rp)
+    first.set_state(psi0)
+    first.solver(1, want_norm=True)
+    first.solver(1, want_norm=True)
+    first.get_norm()
+    first.energy()
+    second = Solver(rp)
+    second.set_state(psi0)
+    first.solver(1, want_norm=True)
+    first.solver(1, want_energy=True)
+    norm = first.solver(1, want_norm=True).norm
+    second.solver(1)
+    np.testing.assert_array_equal(second.get_state(), second_alone)
+    np.testing.assert_array_equal(first.get_state(), alone)
+    # sums of n^3 non-negative terms in two orders: at most n^3 eps apart
+    assert norm == pytest.approx(first.get_norm(), rel=n ** 3 * 2.3e-16)
+    assert first.get_norm() == norm_alone
+    first.close()
+    second.close()
