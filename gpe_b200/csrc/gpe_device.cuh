@@ -963,31 +963,34 @@ __global__ void __launch_bounds__(32 * SITE_TY) k_stage_site(const __grid_consta
   // timeout test (host-armed only): leave without storing, as the march does
   if (*(volatile const int*)a.status == STATUS_EXPIRE_TEST) return;
   if (active) {
+    // ordinary loads: the kernel may be resident before the stage before it
+    // wrote these fields, and a read-only load (ldro) is for data that nobody
+    // writes while the kernel lives; it could also be moved above the wait
     const S* in = (const S*)a.in + o;
     Nb<C> n;
-    n.c0 = to_c<C>(ldro(in));
-    n.xm1 = to_c<C>(ldro(in - 1));
-    n.xp1 = to_c<C>(ldro(in + 1));
-    n.ym1 = to_c<C>(ldro(in - px));
-    n.yp1 = to_c<C>(ldro(in + px));
-    n.zm1 = to_c<C>(ldro(in - pz));
-    n.zp1 = to_c<C>(ldro(in + pz));
+    n.c0 = to_c<C>(in[0]);
+    n.xm1 = to_c<C>(in[-1]);
+    n.xp1 = to_c<C>(in[1]);
+    n.ym1 = to_c<C>(in[-px]);
+    n.yp1 = to_c<C>(in[px]);
+    n.zm1 = to_c<C>(in[-pz]);
+    n.zp1 = to_c<C>(in[pz]);
     if constexpr (R == 2) {
-      n.xm2 = to_c<C>(ldro(in - 2));
-      n.xp2 = to_c<C>(ldro(in + 2));
-      n.ym2 = to_c<C>(ldro(in - 2 * px));
-      n.yp2 = to_c<C>(ldro(in + 2 * px));
-      n.zm2 = to_c<C>(ldro(in - 2 * pz));
-      n.zp2 = to_c<C>(ldro(in + 2 * pz));
+      n.xm2 = to_c<C>(in[-2]);
+      n.xp2 = to_c<C>(in[2]);
+      n.ym2 = to_c<C>(in[-2 * px]);
+      n.yp2 = to_c<C>(in[2 * px]);
+      n.zm2 = to_c<C>(in[-2 * pz]);
+      n.zp2 = to_c<C>(in[2 * pz]);
     } else {
       n.xm2 = n.xp2 = n.ym2 = n.yp2 = n.zm2 = n.zp2 = cx<C>{0, 0};
     }
     S pw[NPWX];
     int q = 0;
-    if constexpr (T::HAS_PSI) pw[q++] = ldro((const S*)a.psi + o);
-    if constexpr (T::HAS_ACC) pw[q++] = ldro((const S*)a.acc + o);
+    if constexpr (T::HAS_PSI) pw[q++] = ((const S*)a.psi)[o];
+    if constexpr (T::HAS_ACC) pw[q++] = ((const S*)a.acc)[o];
 #pragma unroll
-    for (int m = 0; m < T::NK; ++m) pw[q++] = ldro((const S*)a.kin[m] + o);
+    for (int m = 0; m < T::NK; ++m) pw[q++] = ((const S*)a.kin[m])[o];
     pdl_trigger();
     site_stage<S, C, R, KIND>(a, n, pw, i, j, k, o, zghost_pos(k, g.nz, R, a.bcs, a.zghost), cc, r_norm, r_en, r_err);
   }
