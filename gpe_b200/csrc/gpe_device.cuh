@@ -87,8 +87,8 @@ struct alignas(16) StageArgs {
   const void* psi;      // psi_n, read point-wise
   void* acc;            // RK4 accumulator (read/write point-wise)
   void* out;            // stencil output for the next stage (+ ghosts)
-  void* kout;           // Cash-Karp: K_m = dt*f for this stage (stage 6: the largest
-                        // error ratio of the launch so far, as ordered bits, or null)
+  void* kout;           // Cash-Karp: K_m = dt*f for this stage (stage 6: the largest error
+                        // ratio of the launch so far, as ordered bits, or null)
   const void* kin[5];   // Cash-Karp: K_1..K_{m-1}
   double cf_r[2], cf_i[2];  // complex stage coefficients
   double b[6];              // real Cash-Karp coefficients of this stage
@@ -565,14 +565,16 @@ __device__ __forceinline__ bool ck_err_below(const StageArgs& a, cx<double> pd, 
 // free of per-site branches.  MAIN = false stores nothing: the stencil
 // output of each site comes back in ns_out, and the second output of the
 // stage (Q of RK4 stage 2, K_m of Cash-Karp stages 1-5) in aux_out, for
-// callers that store neighbouring sites together.
-template <class S, class C, int R, int KIND, int PY, int NPWX, bool GXY = true, bool GZ = true, bool MAIN = true>
+// callers that store neighbouring sites together.  SCREEN (Cash-Karp stage 6):
+// sites whose error ratio cannot exceed top are not looked at closely.
+template <class S, class C, int R, int KIND, int PY, int NPWX, bool GXY = true, bool GZ = true, bool MAIN = true,
+          bool SCREEN = false>
 __device__ __forceinline__ void sites_update(const StageArgs& a, const cx<C> (&lap)[PY], const cx<C> (&c0)[PY],
                                              const cx<C> (&dpx_in)[PY], const S (&pw)[PY][NPWX],
                                              const bool (&act)[PY], int i, const int (&j)[PY], int k,
                                              const long long (&o)[PY], int gz, const ColumnConsts<C> (&cc)[PY],
                                              double& r_norm, double& r_en, double& r_err, S* ns_out = nullptr,
-                                             S* aux_out = nullptr) {
+                                             S* aux_out = nullptr, double top = 0.0) {
   using T = StageTraits<KIND>;
   const Geom& g = a.g;
   if constexpr (T::FIRST) {
@@ -732,7 +734,8 @@ __device__ __forceinline__ void sites_update(const StageArgs& a, const cx<C> (&l
           const double er = (((DC1 * k1.r + DC3 * k3.r) + DC4 * k4.r) + DC5 * k5.r) + DC6 * Kmd.r;
           const double ei = (((DC1 * k1.i + DC3 * k3.i) + DC4 * k4.i) + DC5 * k5.i) + DC6 * Kmd.i;
           // maxval(abs(err/psi_scal)) of the sites so far; host divides by eps
-          if (act[q] && !ck_err_below(a, pd, k1, er, ei, r_err)) r_err = fmax(r_err, ck_err_ratio(a, pd, k1, er, ei));
+          if (act[q] && !(SCREEN && ck_err_below(a, pd, k1, er, ei, top)))
+            r_err = fmax(r_err, ck_err_ratio(a, pd, k1, er, ei));
         }
       }
     }

@@ -167,17 +167,20 @@ __device__ __forceinline__ TmaRing tma_ring_setup(unsigned char* smem_raw, int* 
 
 // The running maximum of a work item's error ratios (non-negative doubles
 // order as their bits): taken before a plane's sites, given back after them.
-// Single solves start it from the largest ratio of the launch so far, so that
-// away from the worst place hardly a site is looked at twice.
-template <int KIND>
+// It starts from the largest ratio of the launch so far, so that away from the
+// worst place hardly a site is looked at twice.  Single solves only (SCREEN):
+// the solves of a batched launch share no maximum and their items start from
+// zero, and 16 RKF45 solves of 32^3-128^3 took 57.8 ms with the screen, 54.9
+// without (50 steps each).
+template <bool SCREEN>
 __device__ __forceinline__ double take_top(const unsigned long long* s_top, double& r_err) {
-  if constexpr (KIND == K_CK_6)
+  if constexpr (SCREEN)
     r_err = fmax(r_err, __longlong_as_double((long long)*(const volatile unsigned long long*)s_top));
   return r_err;
 }
-template <int KIND>
+template <bool SCREEN>
 __device__ __forceinline__ void put_top(unsigned long long* s_top, double top, double r_err) {
-  if constexpr (KIND == K_CK_6)
+  if constexpr (SCREEN)
     if (r_err > top) atomicMax(s_top, (unsigned long long)__double_as_longlong(r_err));
 }
 
@@ -228,8 +231,10 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
   const int cxp = 2 * (g.xoff + bx * TX);
   const int cyp = by * TY + 2;
 
-  // Cash-Karp stage 6: the item's largest error ratio so far, shared so that
-  // every warp can pass over sites that cannot exceed it (ck_err_below)
+  // Cash-Karp stage 6 of a single solve: the item's largest error ratio so
+  // far, shared so that every warp can pass over sites that cannot exceed it
+  // (ck_err_below)
+  constexpr bool SCREEN = PDL && KIND == K_CK_6;
   __shared__ unsigned long long s_top;
   int issued_s = 0, issued_p = 0;  // meaningful in thread 0 only
   auto issue_stencil = [&](int l) {
@@ -302,7 +307,7 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
     for (int r = 0; r < PY; ++r) q[r][l] = tl[cofs[r]];
   }
   if (!ok) *s_abort = 1;
-  if (KIND == K_CK_6 && tid == 0) s_top = a.kout ? *(volatile const unsigned long long*)a.kout : 0;
+  if (SCREEN && tid == 0) s_top = a.kout ? *(volatile const unsigned long long*)a.kout : 0;
   __syncthreads();
   if (*s_abort) {
     drain(0, 0);
@@ -381,10 +386,11 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
         // after them, by tiles that touch an x/y face and on the first and
         // last R + 1 planes only (uniform branches, the site code stays one)
         S ns[PY];
-        const double top = take_top<KIND>(&s_top, r_err);
-        sites_update<S, C, R, KIND, PY, NPWX, false, false>(a, lap, c0v, dpx, pv, act, i, jr, k, o, gz, cc, r_norm,
-                                                           r_en, r_err, ns);
-        put_top<KIND>(&s_top, top, r_err);
+        const double top = take_top<SCREEN>(&s_top, r_err);
+        sites_update<S, C, R, KIND, PY, NPWX, false, false, true, SCREEN>(a, lap, c0v, dpx, pv, act, i, jr, k, o, gz,
+                                                                        cc, r_norm, r_en, r_err, ns, nullptr,
+                                                                        top);
+        put_top<SCREEN>(&s_top, top, r_err);
         S* out = (S*)a.out;
         if (xyg) {
 #pragma unroll
@@ -424,7 +430,7 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
       if (m + NPS < M) issue_pw(m + NPS);
     }
   }
-  if (KIND == K_CK_6 && tid == 0 && a.kout) atomicMax((unsigned long long*)a.kout, s_top);
+  if (SCREEN && tid == 0 && a.kout) atomicMax((unsigned long long*)a.kout, s_top);
   rg.sbase = SB + L;
   rg.pbase = PB + (NPW > 0 ? M : 0);
   return true;
@@ -494,8 +500,10 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
   const int cxp = 2 * (g.xoff + bx * TX);
   const int cyp = by * TY + 2;
 
-  // Cash-Karp stage 6: the item's largest error ratio so far, shared so that
-  // every warp can pass over sites that cannot exceed it (ck_err_below)
+  // Cash-Karp stage 6 of a single solve: the item's largest error ratio so
+  // far, shared so that every warp can pass over sites that cannot exceed it
+  // (ck_err_below)
+  constexpr bool SCREEN = PDL && KIND == K_CK_6;
   __shared__ unsigned long long s_top;
   int issued_s = 0, issued_p = 0;
   auto issue_stencil = [&](int l) {
@@ -566,7 +574,7 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
     for (int r = 0; r < PY; ++r) q[r][l] = lds_pair(tl + cofs[r]);
   }
   if (!ok) *s_abort = 1;
-  if (KIND == K_CK_6 && tid == 0) s_top = a.kout ? *(volatile const unsigned long long*)a.kout : 0;
+  if (SCREEN && tid == 0) s_top = a.kout ? *(volatile const unsigned long long*)a.kout : 0;
   __syncthreads();
   if (*s_abort) {
     drain(0, 0);
@@ -663,10 +671,10 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
         }
       }
       S ns[NS], ax[NS];
-      const double top = take_top<KIND>(&s_top, r_err);
-      sites_update<S, C, R, KIND, NS, NPWX, false, false, false>(a, lap, c0, dpx, pv, act, i0, jq, k, oq, gz, cc,
-                                                                  r_norm, r_en, r_err, ns, ax);
-      put_top<KIND>(&s_top, top, r_err);
+      const double top = take_top<SCREEN>(&s_top, r_err);
+      sites_update<S, C, R, KIND, NS, NPWX, false, false, false, SCREEN>(a, lap, c0, dpx, pv, act, i0, jq, k, oq, gz, cc,
+                                                                       r_norm, r_en, r_err, ns, ax, top);
+      put_top<SCREEN>(&s_top, top, r_err);
       if constexpr (KIND != K_ENERGY) {
         S* out = (S*)a.out;
 #pragma unroll
@@ -721,7 +729,7 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
       if (m + NPS < M) issue_pw(m + NPS);
     }
   }
-  if (KIND == K_CK_6 && tid == 0 && a.kout) atomicMax((unsigned long long*)a.kout, s_top);
+  if (SCREEN && tid == 0 && a.kout) atomicMax((unsigned long long*)a.kout, s_top);
   rg.sbase = SB + L;
   rg.pbase = PB + (NPW > 0 ? M : 0);
   return true;
