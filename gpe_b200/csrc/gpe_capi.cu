@@ -544,6 +544,11 @@ int enqueue_fixed_step(gpe_handle* h, double dr, double di, bool energy, bool no
   return GPE_OK;
 }
 
+// Can stage 6 screen its error ratios in single precision (ck_err_below)?
+bool ck_screen_holds(double dte_r, double dte_i, double inv_adt) {
+  return dte_r >= 0.0 && hypot(dte_r, dte_i) * inv_adt < 1e3;
+}
+
 // RKF45 = rkqs (src/solve.f90:158-244) with Cash-Karp stages (248-378)
 int rk45_step(gpe_handle* h, gpe_step_info* io, bool energy, bool norm) {
   const gpe_params& p = h->p;
@@ -571,7 +576,7 @@ int rk45_step(gpe_handle* h, gpe_step_info* io, bool energy, bool norm) {
       a.in = ins[m];
       a.out = outs[m];
       for (int q = 0; q < 5; ++q) a.b[q] = 0.0;
-      a.kout = m < 5 ? K[m] : (void*)err_top(h);
+      a.kout = m < 5 ? K[m] : nullptr;
       if (m < 5) {
         for (int q = 0; q <= m; ++q) a.b[q] = CK_B[m][q];
         for (int q = 0; q < m; ++q) a.kin[q] = K[q];
@@ -580,6 +585,7 @@ int rk45_step(gpe_handle* h, gpe_step_info* io, bool energy, bool norm) {
         a.dte_r = dte_r;
         a.dte_i = dte_i;
         a.inv_adt = 1.0 / hypot(dr, di);
+        if (ck_screen_holds(dte_r, dte_i, a.inv_adt)) a.kout = err_top(h);
         a.want_norm = norm;
       }
       a.want_energy = (m == 0 && energy && first);

@@ -88,7 +88,7 @@ struct alignas(16) StageArgs {
   void* acc;            // RK4 accumulator (read/write point-wise)
   void* out;            // stencil output for the next stage (+ ghosts)
   void* kout;           // Cash-Karp: K_m = dt*f for this stage (stage 6: the largest error
-                        // ratio of the launch so far, as ordered bits, or null)
+                        // ratio of the launch so far, as ordered bits; null: no screen)
   const void* kin[5];   // Cash-Karp: K_1..K_{m-1}
   double cf_r[2], cf_i[2];  // complex stage coefficients
   double b[6];              // real Cash-Karp coefficients of this stage
@@ -543,15 +543,19 @@ __device__ __forceinline__ double ck_err_ratio(const StageArgs& a, cx<double> pd
 // largest ratio counts, so most sites can be told apart by single-precision
 // square roots of double-precision squares: the estimate is within 1e-6, the
 // margin 1e-4, and anything outside the range where that holds (or NaN) is
-// not "below".
+// not "below".  Floats under 1e-38 lose digits: bound is formed without the
+// square of top, whose digits would be gone before a large d2 brought it back,
+// and k2 is off by at most 1.1e-23 in |K1| there, 1.1e-5 of a scale above 1e-15
+// while |dt_entry| / |dt| < 1e3 (and dt_entry is not negative: the host sees to
+// both, ck_screen_holds).
 __device__ __forceinline__ bool ck_err_below(const StageArgs& a, cx<double> pd, cx<double> k1, double er, double ei,
                                              double top) {
   const float e2 = (float)(er * er + ei * ei), p2 = (float)(pd.r * pd.r + pd.i * pd.i);
   const float k2 = (float)(k1.r * k1.r + k1.i * k1.i);
   const float fa = sqrtf(k2) * (float)a.inv_adt;
   const float sr = sqrtf(p2) + (float)a.dte_r * fa, si = (float)a.dte_i * fa;
-  const float d2 = sr * sr + si * si, t = (float)top, bound = (t * t) * d2;
-  return e2 * 1.0001f <= bound && bound > 1e-36f && bound < 1e36f && d2 > 1e-30f && d2 < 1e30f && a.dte_r >= 0.0;
+  const float d2 = sr * sr + si * si, t = (float)top, bound = t * (t * d2);
+  return e2 * 1.0001f <= bound && bound > 1e-36f && bound < 1e36f && d2 > 1e-30f && d2 < 1e30f;
 }
 
 // Everything a stage does at the PY interior sites (i, j_q, k) of one thread

@@ -386,7 +386,7 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
         // after them, by tiles that touch an x/y face and on the first and
         // last R + 1 planes only (uniform branches, the site code stays one)
         S ns[PY];
-        const double top = take_top<SCREEN>(&s_top, r_err);
+        const double top = SCREEN && !a.kout ? 0.0 : take_top<SCREEN>(&s_top, r_err);
         sites_update<S, C, R, KIND, PY, NPWX, false, false, true, SCREEN>(a, lap, c0v, dpx, pv, act, i, jr, k, o, gz,
                                                                         cc, r_norm, r_en, r_err, ns, nullptr,
                                                                         top);
@@ -671,7 +671,7 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
         }
       }
       S ns[NS], ax[NS];
-      const double top = take_top<SCREEN>(&s_top, r_err);
+      const double top = SCREEN && !a.kout ? 0.0 : take_top<SCREEN>(&s_top, r_err);
       sites_update<S, C, R, KIND, NS, NPWX, false, false, false, SCREEN>(a, lap, c0, dpx, pv, act, i0, jq, k, oq, gz, cc,
                                                                        r_norm, r_en, r_err, ns, ax, top);
       put_top<SCREEN>(&s_top, top, r_err);
