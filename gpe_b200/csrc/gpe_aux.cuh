@@ -12,7 +12,31 @@ namespace gpe {
 constexpr int ROW_THREADS = 256;
 constexpr int ROW_GRID = 148 * 8;
 
-// f(row k, row j, lane): every interior row once, a warp each
+// Rows shorter than a warp leave lanes idle: their sites go to threads one by
+// one instead, at the price of two divisions a site (in 32 bits where the grid
+// allows it).  set_state of 6 x 1000 x 1000 complex128 240 us by rows, 77 so;
+// 24 x 600 x 600 114, 90.  A second pass over a row with few sites left costs
+// k_pack more than its divisions do (33 x 450 x 450 complex64 74 us by rows, 67
+// by sites; 40 x 500 x 500 91 either way); the other kernels with this rule are
+// faster by rows there already.  Each has an instantiation for either (SITES):
+// one with both loops holds fewer threads.
+constexpr int SHORT_ROW = 32, SHORT_PACK = 40;
+// is a row shorter than a warp, or (up to most sites) little longer?
+inline bool leaves_lanes(const Geom& g, int most) { return g.nx < most && g.nx != 32; }
+inline bool short_rows(const Geom& g) { return g.nx < SHORT_ROW; }
+
+// f(k, j, i, t): every interior site once, t its index in the contiguous array
+template <class F>
+__device__ __forceinline__ void for_each_site(const Geom& g, F f) {
+  const long long n = (long long)g.nx * g.ny * g.nz;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+    const long long r = n <= 0x7fffffff ? (int)t / g.nx : t / g.nx;
+    const int k = (int)(n <= 0x7fffffff ? (int)r / g.ny : r / g.ny);
+    f(k, (int)(r - (long long)k * g.ny), (int)(t - r * g.nx), t);
+  }
+}
+
+// f(k, j, lane, row): every interior row once, a warp each
 template <class F>
 __device__ __forceinline__ void for_each_row(const Geom& g, F f) {
   const int lane = threadIdx.x & 31;
@@ -22,6 +46,14 @@ __device__ __forceinline__ void for_each_row(const Geom& g, F f) {
     const int k = (int)(r / g.ny), j = (int)(r - (long long)k * g.ny);
     f(k, j, lane, r);
   }
+}
+
+// Store a site's value with its face ghosts.
+template <class S>
+__device__ __forceinline__ void put_site(S* __restrict__ f, const Geom& g, int R, int bcs, int zmask, int k, int j,
+                                         int i, S v) {
+  store_with_ghosts(f, g, (long long)(j + 2) * g.px + g.xoff + i, i, j, k, ghost_pos(i, g.nx, R, bcs),
+                    ghost_pos(j, g.ny, R, bcs), zghost_pos(k, g.nz, R, bcs, zmask), v);
 }
 
 // Store a row's values (val(i) for lanes of x) with their face ghosts: whole
@@ -55,22 +87,31 @@ __device__ __forceinline__ void put_row(S* __restrict__ f, const Geom& g, int R,
 // its face ghosts (the halo exchange of gpe.f90:173-176, done once).  256^3
 // complex128: 124 us with an index division per site, 84 us so (82 at the copy
 // rate).
-template <class S, class T2>
+template <bool SITES, class S, class T2>
 __global__ void __launch_bounds__(ROW_THREADS) k_pack(const T2* __restrict__ src, S* __restrict__ dst, Geom g, int R,
-                                                      int bcs, int zmask = 3) {
-  for_each_row(g, [&](int k, int j, int lane, long long r) {
-    const T2* p = src + r * g.nx;
-    put_row(dst, g, R, bcs, zmask, k, j, lane, [&](int i) {
-      const T2 v = p[i];
-      S s;
-      s.x = (typename Stor<S>::R)v.x;
-      s.y = (typename Stor<S>::R)v.y;
-      return s;
+                                                      int bcs, int zmask) {
+  auto conv = [](T2 v) {
+    S s;
+    s.x = (typename Stor<S>::R)v.x;
+    s.y = (typename Stor<S>::R)v.y;
+    return s;
+  };
+  if constexpr (SITES)
+    for_each_site(g, [&](int k, int j, int i, long long t) { put_site(dst, g, R, bcs, zmask, k, j, i, conv(src[t])); });
+  else
+    for_each_row(g, [&](int k, int j, int lane, long long r) {
+      const T2* p = src + r * g.nx;
+      put_row(dst, g, R, bcs, zmask, k, j, lane, [&](int i) { return conv(p[i]); });
     });
-  });
 }
 
-// ghost-padded field -> contiguous interior
+template <class S, class T2>
+void pack(const T2* src, S* dst, const Geom& g, int R, int bcs, int zmask, cudaStream_t st) {
+  if (leaves_lanes(g, SHORT_PACK)) k_pack<true><<<ROW_GRID, ROW_THREADS, 0, st>>>(src, dst, g, R, bcs, zmask);
+  else k_pack<false><<<ROW_GRID, ROW_THREADS, 0, st>>>(src, dst, g, R, bcs, zmask);
+}
+
+// ghost-padded field -> contiguous interior, a warp per row
 template <class S, class T2>
 __global__ void __launch_bounds__(ROW_THREADS) k_unpack(const S* __restrict__ src, T2* __restrict__ dst, Geom g) {
   for_each_row(g, [&](int k, int j, int lane, long long r) {
@@ -85,6 +126,34 @@ __global__ void __launch_bounds__(ROW_THREADS) k_unpack(const S* __restrict__ sr
       p[i] = o;
     }
   });
+}
+
+// the same, a thread per site
+template <class S, class T2>
+__global__ void __launch_bounds__(ROW_THREADS) k_unpack_sites(const S* __restrict__ src, T2* __restrict__ dst, Geom g) {
+  for_each_site(g, [&](int k, int j, int i, long long t) {
+    const S v = src[(long long)(k + 2) * g.pz + (long long)(j + 2) * g.px + g.xoff + i];
+    T2 o;
+    o.x = v.x;
+    o.y = v.y;
+    dst[t] = o;
+  });
+}
+
+// Rows that are short, or long but too few to give every second warp one, are
+// unpacked site by site, six blocks on an SM (40 x 500 x 500 complex128: 79 us
+// by rows, 80, 71, 76 by sites with 8, 6 and 5 blocks; 63 x 350 x 350 62 by
+// rows, 66 by sites; 5000 x 6 x 300 75 by rows, 68 by sites).
+constexpr int SHORT_UNPACK = 48, LONG_UNPACK = 512;
+constexpr int UNPACK_SITES_GRID = 148 * 6;
+
+template <class S, class T2>
+void unpack(const S* src, T2* dst, const Geom& g, cudaStream_t st) {
+  const bool few = g.nx >= LONG_UNPACK && (long long)g.ny * g.nz < ROW_GRID * (ROW_THREADS / 32) / 2;
+  if (few || leaves_lanes(g, SHORT_UNPACK))
+    k_unpack_sites<S, T2><<<UNPACK_SITES_GRID, ROW_THREADS, 0, st>>>(src, dst, g);
+  else
+    k_unpack<S, T2><<<ROW_GRID, ROW_THREADS, 0, st>>>(src, dst, g);
 }
 
 // get_norm partials (variables.f90:554-576): w_i w_j w_k |psi|^2 per block,

@@ -655,15 +655,14 @@ int ensure_staging(gpe_handle* h, size_t bytes) {
 }
 
 int pack_from_device(gpe_handle* h, const void* src, int dtype) {
-  const int nb = ROW_GRID;
   void* dst = h->fields[h->cur];
   const int zm = h->zghost;
   if (h->esz == 16) {
-    if (dtype == GPE_C128) k_pack<double2, double2><<<nb, ROW_THREADS, 0, h->st>>>((const double2*)src, (double2*)dst, h->g, h->R, h->p.bcs, zm);
-    else k_pack<double2, float2><<<nb, ROW_THREADS, 0, h->st>>>((const float2*)src, (double2*)dst, h->g, h->R, h->p.bcs, zm);
+    if (dtype == GPE_C128) pack((const double2*)src, (double2*)dst, h->g, h->R, h->p.bcs, zm, h->st);
+    else pack((const float2*)src, (double2*)dst, h->g, h->R, h->p.bcs, zm, h->st);
   } else {
-    if (dtype == GPE_C128) k_pack<float2, double2><<<nb, ROW_THREADS, 0, h->st>>>((const double2*)src, (float2*)dst, h->g, h->R, h->p.bcs, zm);
-    else k_pack<float2, float2><<<nb, ROW_THREADS, 0, h->st>>>((const float2*)src, (float2*)dst, h->g, h->R, h->p.bcs, zm);
+    if (dtype == GPE_C128) pack((const double2*)src, (float2*)dst, h->g, h->R, h->p.bcs, zm, h->st);
+    else pack((const float2*)src, (float2*)dst, h->g, h->R, h->p.bcs, zm, h->st);
   }
   CU(h, cudaGetLastError());
   CU(h, slab_exchange(h, h->cur));
@@ -671,14 +670,13 @@ int pack_from_device(gpe_handle* h, const void* src, int dtype) {
 }
 
 int unpack_to_device(gpe_handle* h, void* dst, int dtype) {
-  const int nb = ROW_GRID;
   const void* src = h->fields[h->cur];
   if (h->esz == 16) {
-    if (dtype == GPE_C128) k_unpack<double2, double2><<<nb, ROW_THREADS, 0, h->st>>>((const double2*)src, (double2*)dst, h->g);
-    else k_unpack<double2, float2><<<nb, ROW_THREADS, 0, h->st>>>((const double2*)src, (float2*)dst, h->g);
+    if (dtype == GPE_C128) unpack((const double2*)src, (double2*)dst, h->g, h->st);
+    else unpack((const double2*)src, (float2*)dst, h->g, h->st);
   } else {
-    if (dtype == GPE_C128) k_unpack<float2, double2><<<nb, ROW_THREADS, 0, h->st>>>((const float2*)src, (double2*)dst, h->g);
-    else k_unpack<float2, float2><<<nb, ROW_THREADS, 0, h->st>>>((const float2*)src, (float2*)dst, h->g);
+    if (dtype == GPE_C128) unpack((const float2*)src, (double2*)dst, h->g, h->st);
+    else unpack((const float2*)src, (float2*)dst, h->g, h->st);
   }
   CU(h, cudaGetLastError());
   return GPE_OK;

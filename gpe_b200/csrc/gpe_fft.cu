@@ -53,7 +53,7 @@ __device__ __forceinline__ double block_sum(double v, double* scratch) {
 // index division per site, and one read of psi instead of the two of a
 // separate conversion and mass kernel (256^3 complex128: 87 + 121 us for
 // those, 83 for this; bound by HBM, 512 MiB).
-template <class S>
+template <class S, bool SITES>
 __global__ void __launch_bounds__(FFT_THREADS) k_unpack_mass(const S* __restrict__ f, Geom g, double2* __restrict__ a,
                                                              double* part) {
   __shared__ double scratch[32];
@@ -61,7 +61,14 @@ __global__ void __launch_bounds__(FFT_THREADS) k_unpack_mass(const S* __restrict
   const long long rows = (long long)g.ny * g.nz;
   const int tw = gridDim.x * (FFT_THREADS / 32);
   double acc = 0.0;
-  for (long long r = blockIdx.x * (FFT_THREADS / 32) + (threadIdx.x >> 5); r < rows; r += tw) {
+  if constexpr (SITES)
+    for_each_site(g, [&](int k, int j, int i, long long t) {
+      const S v = f[(long long)(k + 2) * g.pz + (long long)(j + 2) * g.px + g.xoff + i];
+      const double x = (double)v.x, y = (double)v.y;
+      a[t] = make_double2(x, y);
+      acc += x * x + y * y;
+    });
+  for (long long r = blockIdx.x * (FFT_THREADS / 32) + (threadIdx.x >> 5); !SITES && r < rows; r += tw) {
     const int k = (int)(r / g.ny), j = (int)(r - (long long)k * g.ny);
     const S* src = f + (long long)(k + 2) * g.pz + (long long)(j + 2) * g.px + g.xoff;
     double2* dst = a + r * g.nx;
@@ -105,6 +112,7 @@ Shells shells() {
 // tot uses the reference's real-space-indexed k grid (kq tables), one term
 // per mode.  256^3: 1004 us with a 32-step lane loop per mode and bin, 112 us
 // so (one read of 256 MiB takes 41; the FP64 divisions of tot bound it).
+template <bool SITES>
 __global__ void __launch_bounds__(FFT_THREADS) k_spectrum(const double2* __restrict__ raw, int nx, int ny, int nz,
                                                           const double* __restrict__ kq, int nbins,
                                                           int want_spectrum, Shells th, double* part) {
@@ -134,7 +142,17 @@ __global__ void __launch_bounds__(FFT_THREADS) k_spectrum(const double2* __restr
     es[q] = 0.0;
     cnt[q] = 0;
   }
-  for (long long u = blockIdx.x * nw + w; u < units; u += tw) {
+  if constexpr (SITES) {  // tot mode by mode where folded rows would leave most lanes idle
+    Geom g = {};
+    g.nx = nx;
+    g.ny = ny;
+    g.nz = nz;
+    for_each_site(g, [&](int k, int j, int i, long long) {
+      const double q = c12 * ((kx[i] + ky[j]) + kz[k]);
+      if (q != 0.0) tot += (q + rho0) / (q * q + 2.0 * rho0 * q);
+    });
+  }
+  for (long long u = blockIdx.x * nw + w; (want_spectrum || !SITES) && u < units; u += tw) {
     const long long row = u / nch;
     const int i = (int)(u - row * nch) * 32 + lane;
     const int kk = (int)(row / (hy + 1)), jj = (int)(row - (long long)kk * (hy + 1));
@@ -156,7 +174,7 @@ __global__ void __launch_bounds__(FFT_THREADS) k_spectrum(const double2* __restr
       const double kx0 = kx[i], kx1 = tx ? kx[nx - i] : 0.0;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        if ((c & 1) >= nj || (c >> 1) >= nk) continue;
+        if (SITES || (c & 1) >= nj || (c >> 1) >= nk) continue;
         const int j = (c & 1) ? ny - jj : jj, k = (c >> 1) ? nz - kk : kk;
         // io.f90:343-360
         const double q0 = c12 * ((kx0 + ky[j]) + kz[k]);
@@ -241,28 +259,37 @@ __global__ void __launch_bounds__(COL_THREADS) k_sum_columns(const double* part,
 
 // raw -> raw (filter max(1 - m k2 / kc^2, 0)) / N (io.f90:567): the factor
 // 1/sqrt(N) of the forward transform and that of the inverse that follows
+template <bool SITES>
 __global__ void __launch_bounds__(FFT_THREADS) k_filter(double2* raw, int nx, int ny, int nz, double mscale, double kc2) {
-  const int lane = threadIdx.x & 31;
   const double n = (double)nx * (double)ny * (double)nz;
-  const long long rows = (long long)ny * nz;
-  const int tw = gridDim.x * (FFT_THREADS / 32);
-  for (long long r = blockIdx.x * (FFT_THREADS / 32) + (threadIdx.x >> 5); r < rows; r += tw) {
-    const int k = (int)(r / ny), j = (int)(r - (long long)k * ny);
-    const int kjk = k2_axis(j, ny) + k2_axis(k, nz);
-    double2* a = raw + r * nx;
+  auto apply = [&](double2* a, int i, int kjk) {
+    const double f = fmax(1.0 - (mscale * (double)(k2_axis(i, nx) + kjk)) / kc2, 0.0) / n;
+    const double2 v = *a;
+    *a = make_double2(v.x * f, v.y * f);
+  };
+  Geom g = {};
+  g.nx = nx;
+  g.ny = ny;
+  g.nz = nz;
+  if constexpr (SITES)
+    for_each_site(g, [&](int k, int j, int i, long long t) { apply(raw + t, i, k2_axis(j, ny) + k2_axis(k, nz)); });
+  else
+    for_each_row(g, [&](int k, int j, int lane, long long r) {
+      const int kjk = k2_axis(j, ny) + k2_axis(k, nz);
 #pragma unroll 4
-    for (int i = lane; i < nx; i += 32) {
-      const double f = fmax(1.0 - (mscale * (double)(k2_axis(i, nx) + kjk)) / kc2, 0.0) / n;
-      const double2 v = a[i];
-      a[i] = make_double2(v.x * f, v.y * f);
-    }
-  }
+      for (int i = lane; i < nx; i += 32) apply(raw + r * nx + i, i, kjk);
+    });
 }
 
 cudaError_t to_contiguous(const Geom& g, int esz, const void* psi_field, double2* buf, double* mpart,
                           cudaStream_t st) {
-  if (esz == 16) k_unpack_mass<double2><<<ROW_BLOCKS, FFT_THREADS, 0, st>>>((const double2*)psi_field, g, buf, mpart);
-  else k_unpack_mass<float2><<<ROW_BLOCKS, FFT_THREADS, 0, st>>>((const float2*)psi_field, g, buf, mpart);
+  const bool sites = short_rows(g);
+  if (esz == 16)
+    (sites ? k_unpack_mass<double2, true> : k_unpack_mass<double2, false>)<<<ROW_BLOCKS, FFT_THREADS, 0, st>>>(
+        (const double2*)psi_field, g, buf, mpart);
+  else
+    (sites ? k_unpack_mass<float2, true> : k_unpack_mass<float2, false>)<<<ROW_BLOCKS, FFT_THREADS, 0, st>>>(
+        (const float2*)psi_field, g, buf, mpart);
   return cudaGetLastError();
 }
 
@@ -307,13 +334,13 @@ cudaError_t fft_condensed(const gpe_params& p, const Geom& g, int esz, const voi
   if (cufftSetStream(plan, st) != CUFFT_SUCCESS) return cudaErrorUnknown;
   if (cufftExecZ2Z(plan, (cufftDoubleComplex*)buf, (cufftDoubleComplex*)buf, CUFFT_FORWARD) != CUFFT_SUCCESS)
     return cudaErrorUnknown;
+  const auto spectrum = short_rows(g) ? k_spectrum<true> : k_spectrum<false>;
   const size_t shm = (size_t)(FFT_THREADS / 32) * nbins * sizeof(double);
   if (shm > 48 * 1024) {
-    e = cudaFuncSetAttribute(k_spectrum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+    e = cudaFuncSetAttribute(spectrum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
     if (e != cudaSuccess) return e;
   }
-  k_spectrum<<<FFT_BLOCKS, FFT_THREADS, shm, st>>>(buf, p.nx, p.ny, p.nz, kq, nbins, want_spectrum ? 1 : 0, shells(),
-                                                   part);
+  spectrum<<<FFT_BLOCKS, FFT_THREADS, shm, st>>>(buf, p.nx, p.ny, p.nz, kq, nbins, want_spectrum ? 1 : 0, shells(), part);
   k_sum_columns<<<width + 1, COL_THREADS, 0, st>>>(part, FFT_BLOCKS, width, mpart, ROW_BLOCKS, sums);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -346,7 +373,8 @@ cudaError_t fft_filtered(const gpe_params& p, const Geom& g, int esz, const void
   if (cufftSetStream(plan, st) != CUFFT_SUCCESS) return cudaErrorUnknown;
   if (cufftExecZ2Z(plan, (cufftDoubleComplex*)buf, (cufftDoubleComplex*)buf, CUFFT_FORWARD) != CUFFT_SUCCESS)
     return cudaErrorUnknown;
-  k_filter<<<ROW_BLOCKS, FFT_THREADS, 0, st>>>(buf, p.nx, p.ny, p.nz, mscale, filter_kc * filter_kc);
+  (short_rows(g) ? k_filter<true> : k_filter<false>)<<<ROW_BLOCKS, FFT_THREADS, 0, st>>>(buf, p.nx, p.ny, p.nz, mscale,
+                                                                                         filter_kc * filter_kc);
   if (cufftExecZ2Z(plan, (cufftDoubleComplex*)buf, (cufftDoubleComplex*)buf, CUFFT_INVERSE) != CUFFT_SUCCESS)
     return cudaErrorUnknown;
   return cudaGetLastError();

@@ -179,23 +179,37 @@ __device__ __forceinline__ bool ic_columnar(const gpe_ic& ic, int q) {
   return (f == GPE_IC_LINE || f == GPE_IC_LINE_PADE) && ic.line.dir == 'z' && ic.line.amp1 == 0.0 && ic.line.amp2 == 0.0;
 }
 
-constexpr int IC_TY = 8;       // rows of a block of 32 x IC_TY columns
+constexpr int IC_THREADS = 256;  // columns of a block
 constexpr int IC_CTAS = 3;     // blocks per SM the registers are fitted to
 constexpr int IC_PLANES = 16;  // most planes a thread takes of its column
 constexpr int IC_MAX = 4;      // factors of a product
 
+// A block is 32 columns along x, or 16 or 8 where x is no longer than that, as
+// many rows of them as it has threads for, or as few as y has, and the rest of
+// its threads are further chunks of planes.
+dim3 ic_block(const Geom& g) {
+  auto fit = [](int n, int most) { return n <= 8 ? 8 : (n <= 16 && most > 16 ? 16 : most); };
+  const int w = fit(g.nx, 32), h = fit(g.ny, IC_THREADS / w < 32 ? IC_THREADS / w : 32);
+  return dim3(w, h, IC_THREADS / (w * h));
+}
+
+// the shape of all but the narrow grids
+bool ic_full(const dim3& b) { return b.x == 32 && b.z == 1; }
+
 // Planes per thread: as many as leave the device IC_CTAS blocks per SM, at
 // most IC_PLANES (beyond that the column's factors cost little anyway).
 int ic_planes(const Geom& g) {
-  const long long tiles = (long long)((g.nx + 31) / 32) * ((g.ny + IC_TY - 1) / IC_TY);
-  const long long chunks = (148LL * IC_CTAS + tiles - 1) / tiles;
+  const dim3 b = ic_block(g);
+  const long long tiles = (long long)((g.nx + b.x - 1) / b.x) * ((g.ny + b.y - 1) / b.y);
+  const long long chunks = (148LL * IC_CTAS + tiles - 1) / tiles * b.z;
   const int z = (int)(g.nz / chunks);
   return z < 1 ? 1 : (z > IC_PLANES ? IC_PLANES : z);
 }
 
 dim3 ic_blocks(const Geom& g) {
-  const int z = ic_planes(g);
-  return dim3((g.nx + 31) / 32, (g.ny + IC_TY - 1) / IC_TY, (g.nz + z - 1) / z);
+  const dim3 b = ic_block(g);
+  const int z = ic_planes(g) * b.z;
+  return dim3((g.nx + b.x - 1) / b.x, (g.ny + b.y - 1) / b.y, (g.nz + z - 1) / z);
 }
 
 // The product of the closed-form factors, taken left to right as the
@@ -207,12 +221,14 @@ dim3 ic_blocks(const Geom& g) {
 // Instruction issue bounds it.  set_ic on 192 x 192 x 384 complex128, us, with
 // every factor (and an arc tangent, a sine and a cosine) per site / so:
 // fermi x line_pade 958 / 72, fermi x line 1104 / 79, ring 1027 / 298.
-template <class S, bool MULT>
+// FULL: blocks of the shape ordinary grids have.
+template <class S, bool MULT, bool FULL>
 __device__ __forceinline__ void ic_column(S* f, const Geom& g, int R, int bcs, const IcGrid& G, const gpe_ic& ic,
                                           int planes, int modulus) {
-  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * IC_TY + threadIdx.y;
+  const int i = blockIdx.x * (FULL ? 32 : blockDim.x) + threadIdx.x;
+  const int j = blockIdx.y * (FULL ? IC_THREADS / 32 : blockDim.y) + threadIdx.y;
   if (i >= g.nx || j >= g.ny) return;
-  const int k0 = blockIdx.z * planes, k1 = min(k0 + planes, g.nz);
+  const int k0 = (FULL ? blockIdx.z : blockIdx.z * blockDim.z + threadIdx.z) * planes, k1 = min(k0 + planes, g.nz);
   const double x = coord(G.xl, G.dx, i), y = coord(G.yl, G.dy, j);
   const double vxy = (G.omx * G.omx) * (x * x) + (G.omy * G.omy) * (y * y);
   double fr[IC_MAX], fi[IC_MAX];
@@ -285,22 +301,22 @@ __device__ __forceinline__ void ic_column(S* f, const Geom& g, int R, int bcs, c
   }
 }
 
-template <class S>
-__global__ void __launch_bounds__(32 * IC_TY, IC_CTAS) k_ic_closed_form(S* f, Geom g, int R, int bcs, IcGrid G,
+template <class S, bool FULL>
+__global__ void __launch_bounds__(IC_THREADS, IC_CTAS) k_ic_closed_form(S* f, Geom g, int R, int bcs, IcGrid G,
                                                                         const __grid_constant__ gpe_ic ic,
                                                                         int planes) {
-  ic_column<S, false>(f, g, R, bcs, G, ic, planes, 0);
+  ic_column<S, false, FULL>(f, g, R, bcs, G, ic, planes, 0);
 }
 
 // psi <- psi * IC (modulus = 0: the state_restart product with init_cond,
 // src/ic.f90:160-162) or psi <- |psi| * IC (modulus = 1:
 // imprint_vortex_line, src/variables.f90:1166-1180), in FP64 per site, the
 // new value stored with its ghosts.
-template <class S>
-__global__ void __launch_bounds__(32 * IC_TY, IC_CTAS) k_ic_multiply(S* f, Geom g, int R, int bcs, IcGrid G,
+template <class S, bool FULL>
+__global__ void __launch_bounds__(IC_THREADS, IC_CTAS) k_ic_multiply(S* f, Geom g, int R, int bcs, IcGrid G,
                                                                      const __grid_constant__ gpe_ic ic, int planes,
                                                                      int modulus) {
-  ic_column<S, true>(f, g, R, bcs, G, ic, planes, modulus);
+  ic_column<S, true, FULL>(f, g, R, bcs, G, ic, planes, modulus);
 }
 
 __device__ __forceinline__ unsigned long long splitmix64(unsigned long long seed, unsigned long long idx) {
@@ -312,26 +328,33 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long seed
 
 // psi_hat(m) = exp(i 2 pi u_m) for |k_m| < kc, else 0; modes in numpy's
 // fftfreq order, u_m from SplitMix64 over the linear mode index
+template <bool SITES>
 __global__ void __launch_bounds__(ROW_THREADS) k_random_spectrum(double2* buf, Geom g, double dx, double dy, double dz,
                                                                  unsigned long long seed, double kc) {
   const int nx = g.nx, ny = g.ny, nz = g.nz;
-  for_each_row(g, [&](int k, int j, int lane, long long r) {
+  auto row2 = [&](int k, int j) {  // ky^2 + kz^2
     const int mj = j < (ny + 1) / 2 ? j : j - ny, mk = k < (nz + 1) / 2 ? k : k - nz;
     const double ky = 2.0 * kPi * mj / (ny * dy), kz = 2.0 * kPi * mk / (nz * dz);
-    const double kyz = kz * kz + ky * ky;
-    for (int i = lane; i < nx; i += 32) {
-      const int mi = i < (nx + 1) / 2 ? i : i - nx;
-      const double kx = 2.0 * kPi * mi / (nx * dx);
-      const long long t = r * nx + i;
-      double2 v = make_double2(0.0, 0.0);
-      if (kyz + kx * kx < kc * kc) {
-        const double u = (double)(splitmix64(seed, (unsigned long long)t) >> 11) * (1.0 / 9007199254740992.0);
-        const double th = 2.0 * kPi * u;
-        v = make_double2(cos(th), sin(th));
-      }
-      buf[t] = v;
+    return kz * kz + ky * ky;
+  };
+  auto mode = [&](double kyz, int i, long long t) {
+    const int mi = i < (nx + 1) / 2 ? i : i - nx;
+    const double kx = 2.0 * kPi * mi / (nx * dx);
+    double2 v = make_double2(0.0, 0.0);
+    if (kyz + kx * kx < kc * kc) {
+      const double u = (double)(splitmix64(seed, (unsigned long long)t) >> 11) * (1.0 / 9007199254740992.0);
+      const double th = 2.0 * kPi * u;
+      v = make_double2(cos(th), sin(th));
     }
-  });
+    buf[t] = v;
+  };
+  if constexpr (SITES)
+    for_each_site(g, [&](int k, int j, int i, long long t) { mode(row2(k, j), i, t); });
+  else
+    for_each_row(g, [&](int k, int j, int lane, long long r) {
+      const double kyz = row2(k, j);
+      for (int i = lane; i < nx; i += 32) mode(kyz, i, r * nx + i);
+    });
 }
 
 // sum |psi|^2 over the buffer (fixed-order block partials, then one block)
@@ -363,22 +386,31 @@ __global__ void __launch_bounds__(256) k_sum_parts(double* part, int nb) {
 }
 
 // psi = buf * sqrt(n / sum|buf|^2) into the padded field with ghosts
-template <class S>
+template <bool SITES, class S>
 __global__ void __launch_bounds__(ROW_THREADS) k_pack_scaled(const double2* __restrict__ buf,
                                                              const double* __restrict__ total, S* f, Geom g, int R,
                                                              int bcs) {
   const double n = (double)g.nx * (double)g.ny * (double)g.nz;
   const double sc = 1.0 / sqrt(*total / n);
-  for_each_row(g, [&](int k, int j, int lane, long long r) {
-    const double2* p = buf + r * g.nx;
-    put_row(f, g, R, bcs, 3, k, j, lane, [&](int i) {
-      const double2 v = p[i];
-      S s;
-      s.x = (typename Stor<S>::R)(v.x * sc);
-      s.y = (typename Stor<S>::R)(v.y * sc);
-      return s;
+  auto scaled = [&](double2 v) {
+    S s;
+    s.x = (typename Stor<S>::R)(v.x * sc);
+    s.y = (typename Stor<S>::R)(v.y * sc);
+    return s;
+  };
+  if constexpr (SITES)
+    for_each_site(g, [&](int k, int j, int i, long long t) { put_site(f, g, R, bcs, 3, k, j, i, scaled(buf[t])); });
+  else
+    for_each_row(g, [&](int k, int j, int lane, long long r) {
+      const double2* p = buf + r * g.nx;
+      put_row(f, g, R, bcs, 3, k, j, lane, [&](int i) { return scaled(p[i]); });
     });
-  });
+}
+
+template <class S>
+void pack_scaled(const double2* buf, const double* total, S* f, const Geom& g, int R, int bcs, cudaStream_t st) {
+  if (short_rows(g)) k_pack_scaled<true><<<ROW_GRID, ROW_THREADS, 0, st>>>(buf, total, f, g, R, bcs);
+  else k_pack_scaled<false><<<ROW_GRID, ROW_THREADS, 0, st>>>(buf, total, f, g, R, bcs);
 }
 
 // 3-D Z2Z plans, one per (device, grid), created on first use
@@ -468,20 +500,29 @@ cudaError_t ic_multiply(const gpe_params& p, const Geom& g, int esz, int R, cons
                         int modulus, cudaStream_t st) {
   if (ic_needs_fft(&ic)) return cudaErrorInvalidValue;
   const IcGrid G = ic_grid(p);
-  const dim3 nb = ic_blocks(g), nt(32, IC_TY);
-  if (esz == 16) k_ic_multiply<double2><<<nb, nt, 0, st>>>((double2*)psi_field, g, R, p.bcs, G, ic, ic_planes(g), modulus);
-  else k_ic_multiply<float2><<<nb, nt, 0, st>>>((float2*)psi_field, g, R, p.bcs, G, ic, ic_planes(g), modulus);
+  const dim3 nb = ic_blocks(g), nt = ic_block(g);
+  const bool full = ic_full(nt);
+  if (esz == 16)
+    (full ? k_ic_multiply<double2, true> : k_ic_multiply<double2, false>)<<<nb, nt, 0, st>>>(
+        (double2*)psi_field, g, R, p.bcs, G, ic, ic_planes(g), modulus);
+  else
+    (full ? k_ic_multiply<float2, true> : k_ic_multiply<float2, false>)<<<nb, nt, 0, st>>>(
+        (float2*)psi_field, g, R, p.bcs, G, ic, ic_planes(g), modulus);
   return cudaGetLastError();
 }
 
 cudaError_t ic_generate(const gpe_params& p, const Geom& g, int esz, int R, const gpe_ic& ic, void* psi_field,
                         void* work, size_t work_bytes, cudaStream_t st) {
   const IcGrid G = ic_grid(p);
-  const int nb = ROW_GRID;
   if (!ic_needs_fft(&ic)) {
-    const dim3 cb = ic_blocks(g), nt(32, IC_TY);
-    if (esz == 16) k_ic_closed_form<double2><<<cb, nt, 0, st>>>((double2*)psi_field, g, R, p.bcs, G, ic, ic_planes(g));
-    else k_ic_closed_form<float2><<<cb, nt, 0, st>>>((float2*)psi_field, g, R, p.bcs, G, ic, ic_planes(g));
+    const dim3 nb = ic_blocks(g), nt = ic_block(g);
+    const bool full = ic_full(nt);
+    if (esz == 16)
+      (full ? k_ic_closed_form<double2, true> : k_ic_closed_form<double2, false>)<<<nb, nt, 0, st>>>(
+          (double2*)psi_field, g, R, p.bcs, G, ic, ic_planes(g));
+    else
+      (full ? k_ic_closed_form<float2, true> : k_ic_closed_form<float2, false>)<<<nb, nt, 0, st>>>(
+          (float2*)psi_field, g, R, p.bcs, G, ic, ic_planes(g));
     return cudaGetLastError();
   }
   const long long n = (long long)p.nx * p.ny * p.nz;
@@ -489,7 +530,8 @@ cudaError_t ic_generate(const gpe_params& p, const Geom& g, int esz, int R, cons
   if (!work || work_bytes < need) return cudaErrorInvalidValue;
   double2* buf = (double2*)work;
   double* part = (double*)((char*)work + (((size_t)n * sizeof(double2) + 255) & ~size_t(255)));
-  k_random_spectrum<<<nb, ROW_THREADS, 0, st>>>(buf, g, G.dx, G.dy, G.dz, (unsigned long long)ic.seed, ic.kc);
+  (short_rows(g) ? k_random_spectrum<true> : k_random_spectrum<false>)<<<ROW_GRID, ROW_THREADS, 0, st>>>(
+      buf, g, G.dx, G.dy, G.dz, (unsigned long long)ic.seed, ic.kc);
   cufftHandle plan;
   if (!plan_for(p.nx, p.ny, p.nz, &plan)) return cudaErrorUnknown;
   if (cufftSetStream(plan, st) != CUFFT_SUCCESS) return cudaErrorUnknown;
@@ -498,8 +540,8 @@ cudaError_t ic_generate(const gpe_params& p, const Geom& g, int esz, int R, cons
   const int nbs = 1000;
   k_sumsq<<<nbs, 256, 0, st>>>(buf, n, part);
   k_sum_parts<<<1, 256, 0, st>>>(part, nbs);
-  if (esz == 16) k_pack_scaled<double2><<<nb, ROW_THREADS, 0, st>>>(buf, part + nbs, (double2*)psi_field, g, R, p.bcs);
-  else k_pack_scaled<float2><<<nb, ROW_THREADS, 0, st>>>(buf, part + nbs, (float2*)psi_field, g, R, p.bcs);
+  if (esz == 16) pack_scaled(buf, part + nbs, (double2*)psi_field, g, R, p.bcs, st);
+  else pack_scaled(buf, part + nbs, (float2*)psi_field, g, R, p.bcs, st);
   return cudaGetLastError();
 }
 

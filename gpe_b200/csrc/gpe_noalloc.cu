@@ -16,7 +16,7 @@
 // it is only a stand-in symbol.  The first call on each device, with that
 // device current, looks up the real device address with
 // cudaGetSymbolAddress and caches it per device; kernels get that pointer.
-// The same first call loads both dtype instances of the reduction kernel on
+// The same first call loads all instances of the reduction kernel on
 // that device (cudaFuncGetAttributes), so with lazy module loading no later
 // call loads code; make it before any stream capture.  The cached address is
 // not refreshed after cudaDeviceReset or a primary-context reset, which this
@@ -80,8 +80,10 @@ int plane_parts(int ny, int nz) {
 // lanes along x, then a tree), so results are deterministic.  A warp walks
 // whole rows, two at a time: no index division, and a plane is spread over as many blocks as the chip wants.  192 x 192 x 384
 // complex128 (216 MiB): 97 us with one 256-thread block per plane and a
-// 64-bit division per site, 46 us so (35 at the copy rate).
-template <class T2>
+// 64-bit division per site, 46 us so (35 at the copy rate).  SITES: rows shorter
+// than a warp, whose sites go to threads one by one (6 x 1000 x 1000 complex128
+// 98 us by rows, 41 so).
+template <class T2, bool SITES>
 __global__ void __launch_bounds__(kThreads) k_plane_sums(const T2* __restrict__ psi, int nx, int ny, int parts,
                                                          double* scratch) {
   __shared__ double red[kThreads / 32];
@@ -90,7 +92,20 @@ __global__ void __launch_bounds__(kThreads) k_plane_sums(const T2* __restrict__ 
   const int j0 = (int)((long long)ny * b / parts), j1 = (int)((long long)ny * (b + 1) / parts);
   double s = 0.0;
   constexpr int kW = kThreads / 32;
-  for (int j = j0 + w; j < j1; j += 2 * kW) {
+  if constexpr (SITES) {
+    // a 32-bit division each: a part holds a 1184th of what fits on the device,
+    // or a few rows
+    const T2* p = psi + ((long long)k * ny + j0) * nx;
+    const int n = (j1 - j0) * nx;
+#pragma unroll 4
+    for (int t = threadIdx.x; t < n; t += kThreads) {
+      const int j = t / nx;
+      const T2 v = p[t];
+      const double re = (double)v.x, im = (double)v.y;
+      s += (quad_weight(t - j * nx, nx) * quad_weight(j0 + j, ny)) * (re * re + im * im);
+    }
+  }
+  for (int j = j0 + w; !SITES && j < j1; j += 2 * kW) {
     // two rows at a time: eight loads in flight per lane
     const bool two = j + kW < j1;
     const T2* p = psi + ((long long)k * ny + j) * nx;
@@ -141,7 +156,7 @@ int reject(const char* why) {
 }
 
 // Set-up of the current device (once): the scratch array's device address,
-// and both reduction kernels loaded.  Returns nullptr on a CUDA error.
+// and the reduction kernels loaded.  Returns nullptr on a CUDA error.
 double* scratch_of(int dev) {
   double* p = g_scratch_addr[dev].load(std::memory_order_acquire);
   if (p) return p;
@@ -151,8 +166,10 @@ double* scratch_of(int dev) {
   void* addr = nullptr;
   if (cudaGetSymbolAddress(&addr, g_norm_scratch) != cudaSuccess || !addr) return nullptr;
   cudaFuncAttributes fa;
-  if (cudaFuncGetAttributes(&fa, k_plane_sums<double2>) != cudaSuccess ||
-      cudaFuncGetAttributes(&fa, k_plane_sums<float2>) != cudaSuccess ||
+  if (cudaFuncGetAttributes(&fa, k_plane_sums<double2, false>) != cudaSuccess ||
+      cudaFuncGetAttributes(&fa, k_plane_sums<double2, true>) != cudaSuccess ||
+      cudaFuncGetAttributes(&fa, k_plane_sums<float2, false>) != cudaSuccess ||
+      cudaFuncGetAttributes(&fa, k_plane_sums<float2, true>) != cudaSuccess ||
       cudaFuncGetAttributes(&fa, k_plane_total) != cudaSuccess)
     return nullptr;
   p = (double*)addr;
@@ -179,10 +196,13 @@ extern "C" int gpe_norm_noalloc(const void* psi_dev, int32_t dtype, int32_t nx, 
   if (!scratch) return GPE_ERR_CUDA;
   cudaStream_t st = (cudaStream_t)stream;
   const int parts = plane_parts(ny, nz);
+  const bool sites = nx < 32;
   if (dtype == GPE_C128)
-    k_plane_sums<double2><<<nz * parts, kThreads, 0, st>>>((const double2*)psi_dev, nx, ny, parts, scratch);
+    (sites ? k_plane_sums<double2, true> : k_plane_sums<double2, false>)<<<nz * parts, kThreads, 0, st>>>(
+        (const double2*)psi_dev, nx, ny, parts, scratch);
   else
-    k_plane_sums<float2><<<nz * parts, kThreads, 0, st>>>((const float2*)psi_dev, nx, ny, parts, scratch);
+    (sites ? k_plane_sums<float2, true> : k_plane_sums<float2, false>)<<<nz * parts, kThreads, 0, st>>>(
+        (const float2*)psi_dev, nx, ny, parts, scratch);
   k_plane_total<<<1, kThreads, 0, st>>>(scratch, nz, parts, dx, dy, dz, norm_dev);
   return cudaGetLastError() == cudaSuccess ? GPE_OK : GPE_ERR_CUDA;
 }

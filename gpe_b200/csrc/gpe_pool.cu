@@ -277,11 +277,9 @@ int upload_state(gpe_pool* P, Solve* s, const void* psi) {
   void* stage = s->f[1];  // free until the first step
   PCU(P, cudaMemcpyAsync(stage, psi, s->interior_bytes(), cudaMemcpyHostToDevice, P->st));
   if (s->esz == 16)
-    k_pack<double2, double2><<<ROW_GRID, ROW_THREADS, 0, P->st>>>((const double2*)stage, (double2*)s->f[0], s->g, s->R,
-                                                                  s->p.bcs);
+    pack((const double2*)stage, (double2*)s->f[0], s->g, s->R, s->p.bcs, 3, P->st);
   else
-    k_pack<float2, float2><<<ROW_GRID, ROW_THREADS, 0, P->st>>>((const float2*)stage, (float2*)s->f[0], s->g, s->R,
-                                                                s->p.bcs);
+    pack((const float2*)stage, (float2*)s->f[0], s->g, s->R, s->p.bcs, 3, P->st);
   PCU(P, cudaGetLastError());
   return GPE_OK;
 }
@@ -289,9 +287,9 @@ int upload_state(gpe_pool* P, Solve* s, const void* psi) {
 int download_state(gpe_pool* P, Solve* s, int fidx) {
   void* stage = s->f[2];  // a stage field: the solve is done stepping
   if (s->esz == 16)
-    k_unpack<double2, double2><<<ROW_GRID, ROW_THREADS, 0, P->st>>>((const double2*)s->f[fidx], (double2*)stage, s->g);
+    unpack((const double2*)s->f[fidx], (double2*)stage, s->g, P->st);
   else
-    k_unpack<float2, float2><<<ROW_GRID, ROW_THREADS, 0, P->st>>>((const float2*)s->f[fidx], (float2*)stage, s->g);
+    unpack((const float2*)s->f[fidx], (float2*)stage, s->g, P->st);
   PCU(P, cudaGetLastError());
   PCU(P, cudaMemcpyAsync(s->out, stage, s->interior_bytes(), cudaMemcpyDeviceToHost, P->st));
   return GPE_OK;
