@@ -189,7 +189,7 @@ struct NormSolve {
 struct NormItem {
   int solve, k0;
 };
-constexpr int NORM_PLANES = 4;
+constexpr int NORM_PLANES = 1;  // (a warp's rows are a serial chain of loads)
 
 template <class S>
 __global__ void __launch_bounds__(ROW_THREADS) k_norm_batch(const NormSolve* __restrict__ sv,

@@ -463,8 +463,11 @@ int ensure_stream(gpe_pool* P, Class& c) {
   return GPE_OK;
 }
 
-// Queue the norms of the class's solves (their current states) on its stream.
-int norms_enqueue(gpe_pool* P, int cm, int fam) {
+// Work list and table of the norms of the class's solves (their current
+// states).  The class's stream is idle, and no class's steps are queued yet the
+// first time: what has to wait or allocate does so before there is work to wait
+// for.  Later only the states' addresses can have changed (RKF45).
+int norms_prepare(gpe_pool* P, int cm, int fam) {
   Class& c = P->cls[cm][fam];
   const int ns = (int)c.solves.size();
   if (int rc = ensure_stream(P, c)) return rc;
@@ -472,8 +475,10 @@ int norms_enqueue(gpe_pool* P, int cm, int fam) {
   PCU(P, c.hnsolve.ensure(ns));
   PCU(P, c.nres.ensure((size_t)ns * RED_SLOTS));
   PCU(P, c.hnres.ensure((size_t)ns * RED_SLOTS));
+  bool moved = false;
   if (c.norm_for != c.solves) {
     PCU(P, cudaStreamSynchronize(c.st));
+    moved = true;
     c.hnitem.clear();
     c.hnfirst.assign(1, 0);
     for (int q = 0; q < ns; ++q) {
@@ -492,9 +497,19 @@ int norms_enqueue(gpe_pool* P, int cm, int fam) {
   for (int q = 0; q < ns; ++q) {
     const Solve* s = c.solves[q];
     const double* w = s->tables + 2 * ((size_t)s->g.nx + s->g.ny + s->g.nz);
+    if (!moved && c.hnsolve.p[q].psi == s->f[s->cur]) continue;
     c.hnsolve.p[q] = NormSolve{s->g, w, w + s->g.nx, w + s->g.nx + s->g.ny, s->f[s->cur]};
+    moved = true;
   }
-  PCU(P, cudaMemcpyAsync(c.nsolve.p, c.hnsolve.p, ns * sizeof(NormSolve), cudaMemcpyHostToDevice, c.st));
+  if (moved)
+    PCU(P, cudaMemcpyAsync(c.nsolve.p, c.hnsolve.p, ns * sizeof(NormSolve), cudaMemcpyHostToDevice, c.st));
+  return GPE_OK;
+}
+
+// Queue the norms on the class's stream.
+int norms_enqueue(gpe_pool* P, int cm, int fam) {
+  Class& c = P->cls[cm][fam];
+  const int ns = (int)c.solves.size();
   const int nb = (int)c.hnitem.size();
   if (class_cmode(cm) == CM_F64) k_norm_batch<double2><<<nb, ROW_THREADS, 0, c.st>>>(c.nsolve.p, c.nitem.p, c.npart.p);
   else k_norm_batch<float2><<<nb, ROW_THREADS, 0, c.st>>>(c.nsolve.p, c.nitem.p, c.npart.p);
@@ -809,9 +824,13 @@ int gpe_pool_step(gpe_pool* P, int64_t max_steps, int32_t* n_active) {
     for (Solve* s : c.solves) chunk = std::min(chunk, s->nsteps - s->done);
     if (!c.solves.empty() && chunk > 0) {
       if (int rc = rk4_prepare(P, cm)) return rc;
+      if (int rc = norms_prepare(P, cm, FAM_RK4)) return rc;
       chunks[cm] = chunk;
     }
   }
+  for (int cm = 0; cm < NCLS; ++cm)
+    if (!P->cls[cm][FAM_RK45].solves.empty())
+      if (int rc = norms_prepare(P, cm, FAM_RK45)) return rc;
   // step by step over the classes, so that each class's stream has work while
   // the host is busy with the others
   const int64_t longest = *std::max_element(chunks, chunks + NCLS);
@@ -840,12 +859,18 @@ int gpe_pool_step(gpe_pool* P, int64_t max_steps, int32_t* n_active) {
       if (!sv[cm].empty())
         if (int rc = rk45_collect(P, cm, sv[cm])) return rc;
   }
-  for (int cm = 0; cm < NCLS; ++cm)
-    if (!P->cls[cm][FAM_RK45].solves.empty())
-      if (int rc = norms_enqueue(P, cm, FAM_RK45)) return rc;
+  // (their norms are wanted with their results only: error norms tell of states
+  // that blew up)
+  bool want[NCLS] = {false};
+  for (int cm = 0; cm < NCLS; ++cm) {
+    for (Solve* s : P->cls[cm][FAM_RK45].solves) want[cm] |= s->done >= s->nsteps || s->status != GPE_OK;
+    if (!want[cm]) continue;
+    if (int rc = norms_prepare(P, cm, FAM_RK45)) return rc;
+    if (int rc = norms_enqueue(P, cm, FAM_RK45)) return rc;
+  }
   for (int cm = 0; cm < NCLS; ++cm) {
     Class& c = P->cls[cm][FAM_RK45];
-    if (c.solves.empty()) continue;
+    if (!want[cm]) continue;
     PCU(P, cudaStreamSynchronize(c.st));
     for (size_t q = 0; q < c.solves.size(); ++q)
       if (c.solves[q]->done > 0) c.solves[q]->norm = norm_of(c, (int)q);
