@@ -377,8 +377,19 @@ void rk45_tables(gpe_pool* P, Solve* s, BatchStage* t6) {
 // 16 solves of 32^3-128^3 in five classes took 16.0 ms for 40 steps with
 // items of up to 64 planes (46 to 132 of them in a launch for 592 slots) and
 // take 9.2 so; one 96^3 solve runs at 17 instead of 3.5 G site-updates/s.
+// The classes of a family run side by side, so the others' work helps to fill
+// the device, though not all of it: launches of different classes meet as they
+// come.  Counting 0.3 to 0.5 of it is best, nothing of it picks items too short
+// (30 solves of 32^3-128^3 in three classes, 60 steps: 42.3 ms with none, 40.5
+// with 0.3 and 0.5, 40.5 with fixed items of 64; 16 of 24^3-64^3 in five classes
+// 7.06, 6.06, 5.94, 14.2; all of it 12.1 against 9.2 ms on the first mix above).
 // States do not depend on the items.
-void choose_items(int cm, int fam, const std::vector<Solve*>& sv) {
+constexpr double OTHERS_SHARE = 0.4;
+void choose_items(gpe_pool* P, int cm, int fam, const std::vector<Solve*>& sv) {
+  double others = 0.0;
+  for (int oc = 0; oc < NCLS; ++oc)
+    if (oc != cm)
+      for (const Solve* s : P->cls[oc][fam].solves) others += (double)s->ntx * s->nty * s->g.nz;
   int occ = 0;
   BatchLaunch q{};
   q.ns = (int)sv.size();
@@ -395,7 +406,7 @@ void choose_items(int cm, int fam, const std::vector<Solve*>& sv) {
       work += (double)s->ntx * s->nty * (s->g.nz + (double)n * lead);
       longest = std::max(longest, (double)zc + lead);
     }
-    const double t = std::max(longest, work / slots + 0.1 * longest);
+    const double t = std::max(longest, (work + OTHERS_SHARE * others) / slots + 0.1 * longest);
     if (best_t == 0.0 || t < best_t) {
       best = z;
       best_t = t;
@@ -410,7 +421,7 @@ void choose_items(int cm, int fam, const std::vector<Solve*>& sv) {
 // Work list of the given solves (in order) into the class buffers.
 int build_items(gpe_pool* P, int cm, int fam, const std::vector<Solve*>& sv) {
   Class& c = P->cls[cm][fam];
-  choose_items(cm, fam, sv);
+  choose_items(P, cm, fam, sv);
   c.built_for = sv;
   c.hitems.clear();
   c.hfirst.assign(1, 0);
