@@ -78,14 +78,15 @@ int zc_from_env(int nz) {
 // worst) and 15 % faster than a fixed target of 8 CTAs per SM.
 int balanced_zc(const Geom& g, int esz, int R, long long tiles, long long slots) {
   const double lead = 5 * R - 4;
-  const int zmax = std::min(g.nz, esz >= 16 ? 24 : 20);
-  int best = 1;
+  const int zmin = (g.nz + GRID_YZ_MAX - 1) / GRID_YZ_MAX;  // what one launch can hold
+  const int zmax = std::max(zmin, std::min(g.nz, esz >= 16 ? 24 : 20));
+  int best = zmin;
   double best_cost = 0.0;
-  for (int z = 1; z <= zmax; ++z) {
+  for (int z = zmin; z <= zmax; ++z) {
     const double x = (double)(tiles * ((g.nz + z - 1) / z)) / (double)slots, whole = ceil(x);
     const double rounds = x <= 1.0 ? 1.0 : x + 0.3 + (whole - x - 0.3) * pow(0.5, whole - 1.0);
     const double cost = rounds * (z + lead) * (1.0 + 0.004 * z);
-    if (z == 1 || cost < best_cost) {
+    if (z == zmin || cost < best_cost) {
       best = z;
       best_cost = cost;
     }

@@ -22,6 +22,8 @@ void param_layout(const gpe_params* p, Geom& g, int& esz);
 long long padded_elems(const Geom& g);
 // fields a scheme keeps per solve
 int scheme_fields(int scheme);
+// most blocks of a launch along y and along z
+constexpr int GRID_YZ_MAX = 65535;
 // z planes per CTA asked for in the environment (GPE_ZC), 0 = none
 int zc_from_env(int nz);
 // z planes per CTA of a stage launch over `tiles` x-y tiles when `slots` CTAs

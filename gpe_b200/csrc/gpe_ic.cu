@@ -12,6 +12,7 @@
 #include <tuple>
 
 #include "gpe_aux.cuh"
+#include "gpe_common.h"
 #include "gpe_ic.h"
 
 namespace gpe {
@@ -186,10 +187,12 @@ constexpr int IC_MAX = 4;      // factors of a product
 
 // A block is 32 columns along x, or 16 or 8 where x is no longer than that, as
 // many rows of them as it has threads for, or as few as y has, and the rest of
-// its threads are further chunks of planes.
+// its threads are further chunks of planes.  (A y too long for a launch's blocks
+// of few rows gets blocks of many.)
 dim3 ic_block(const Geom& g) {
   auto fit = [](int n, int most) { return n <= 8 ? 8 : (n <= 16 && most > 16 ? 16 : most); };
-  const int w = fit(g.nx, 32), h = fit(g.ny, IC_THREADS / w < 32 ? IC_THREADS / w : 32);
+  const bool long_y = g.ny > GRID_YZ_MAX * (IC_THREADS / 32);
+  const int w = long_y ? 8 : fit(g.nx, 32), h = fit(g.ny, IC_THREADS / w < 32 ? IC_THREADS / w : 32);
   return dim3(w, h, IC_THREADS / (w * h));
 }
 
@@ -197,13 +200,14 @@ dim3 ic_block(const Geom& g) {
 bool ic_full(const dim3& b) { return b.x == 32 && b.z == 1; }
 
 // Planes per thread: as many as leave the device IC_CTAS blocks per SM, at
-// most IC_PLANES (beyond that the column's factors cost little anyway).
+// most IC_PLANES (beyond that the column's factors cost little anyway) or what
+// one launch needs to reach the end of z.
 int ic_planes(const Geom& g) {
   const dim3 b = ic_block(g);
   const long long tiles = (long long)((g.nx + b.x - 1) / b.x) * ((g.ny + b.y - 1) / b.y);
   const long long chunks = (148LL * IC_CTAS + tiles - 1) / tiles * b.z;
-  const int z = (int)(g.nz / chunks);
-  return z < 1 ? 1 : (z > IC_PLANES ? IC_PLANES : z);
+  const int z = (int)(g.nz / chunks), least = (int)((g.nz - 1) / (GRID_YZ_MAX * (long long)b.z)) + 1;
+  return z > IC_PLANES ? (least > IC_PLANES ? least : IC_PLANES) : (z < least ? least : z);
 }
 
 dim3 ic_blocks(const Geom& g) {
