@@ -1077,7 +1077,8 @@ static int step_impl(gpe_handle* h, int64_t nsteps, gpe_step_info* io, bool wait
     // kernel has been loaded and configured.  The graph of GRAPH_STEPS steps is
     // captured for long calls, else when a dt comes again; that of a step with
     // a norm when the last one had the same dt (a relaxation asks for one per
-    // call)
+    // call).  A call that does not wait has no use for the results' copy, and
+    // its stream may be its owner's to capture: its normed step runs plainly
     const bool can = use_step_graphs(h), graphs = can && nsteps >= 3;
     const bool again = same_dt(h->call_dt, dr, di);
     const bool have = have_step_graph(h, 0, dr, di) || have_step_graph(h, 1, dr, di);
@@ -1091,7 +1092,7 @@ static int step_impl(gpe_handle* h, int64_t nsteps, gpe_step_info* io, bool wait
         if (int rc = ensure_step_graph(h, which, dr, di)) return rc;
         CU(h, cudaGraphLaunch(h->step_graph[which], h->st));
         if (which) took = GRAPH_STEPS;
-      } else if (can && n && !e && same_dt(h->norm_dt, dr, di)) {
+      } else if (can && wait && n && !e && same_dt(h->norm_dt, dr, di)) {
         if (int rc = ensure_step_graph(h, 2, dr, di)) return rc;
         CU(h, cudaGraphLaunch(h->step_graph[2], h->st));
         copied = true;
