@@ -56,7 +56,7 @@ def time_rk4(rp: RunParams, steps: int = 20, target_sites: int = 32 << 20) -> fl
     psi = np.ones((rp.nz, rp.ny, rp.nx), np.complex64 if rp.storage == "c64" else np.complex128)
     for c in range(copies):
         pool.submit(rp, psi, steps + 4, c)
-    pool.step(3)  # joins the batch, captures the step graph
+    pool.step(3)  # joins the batch; kernels loaded, work lists made
     t0 = time.perf_counter()
     pool.step(steps)
     t = time.perf_counter() - t0
@@ -111,7 +111,7 @@ def time_mix(params, states, cap: int, steps: int = 20) -> float:
     pool = Pool(sum(Pool.solve_bytes(p) for p in runs) + (256 << 20))
     for k, (p, psi) in enumerate(zip(runs, states)):
         assert pool.submit(p, psi, steps + 4, k)
-    pool.step(3)  # joins the batch, captures the step graph
+    pool.step(3)  # joins the batch; kernels loaded, work lists made
     t0 = time.perf_counter()
     pool.step(steps)
     t = time.perf_counter() - t0

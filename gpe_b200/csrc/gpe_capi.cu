@@ -3,9 +3,9 @@
 // One handle = one solve (or one z-slab of a decomposed solve): ghost-padded
 // device fields, per-axis tables, a stream, reduction buffers.  gpe_step()
 // enqueues one fused stage kernel per Runge-Kutta stage (steps without
-// reductions as a replayed graph of one step); the time bookkeeping follows
-// the reference's solver() routines (src/solve.f90:57-244) on the host, in
-// FP64.
+// reductions as replayed graphs of eight steps and of one, a step with a norm
+// that comes again as a graph of its own); the time bookkeeping follows the
+// reference's solver() routines (src/solve.f90:57-244) on the host, in FP64.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
@@ -119,10 +119,10 @@ struct gpe_handle {
   cudaStream_t snap_st = nullptr;
   cudaEvent_t snap_ready = nullptr, snap_done = nullptr;
   bool snap_pending = false;
-  // one captured RK4/RK2 step without reductions, replayed by gpe_step
-  // (the stage arguments, dt included, are baked into the graph)
-  // [0] holds one step, [1] GRAPH_STEPS of them, so that a long run pays a
-  // graph launch and its gap once per GRAPH_STEPS steps; [2] one step with
+  // captured RK4/RK2 steps, replayed by gpe_step (the stage arguments, dt
+  // included, and the addresses they hold are baked into a graph): [0] one
+  // step without reductions, [1] GRAPH_STEPS of them, so that a long run pays
+  // a graph launch and its gap once per GRAPH_STEPS steps, [2] one step with
   // the norm of its result and the copy of the results to the host
   cudaGraphExec_t step_graph[3] = {nullptr, nullptr, nullptr};
   double graph_dt[3][2] = {};  // the dt of each

@@ -7,7 +7,10 @@
 // class keeps a work list of (solve, tile, z-chunk) items and a device table
 // of per-solve stage arguments and tensor maps.  One persistent launch of
 // k_stage_batch per Runge-Kutta stage advances every solve of a class, each
-// class on its own stream, the host taking the classes step by step in turn.
+// class on its own stream.  The host queues the RK4 classes' steps of a call
+// first, step by step over the classes in turn, and then takes the RKF45
+// classes through their attempts: those run beside what of the RK4 steps is
+// still queued, which is little where a call's steps fill the launch queue.
 // (Replayed step graphs kept the host in the launch of a class's next step
 // until the one before it was done, so the classes ran one after another.)
 // RKF45 solves share their attempts: after each attempt every solve's error

@@ -841,8 +841,8 @@ int main(int argc, char** argv) {
   imprint.factor[0] = GPE_IC_LINE;
   imprint.line = c.P.vl1;
   // Fixed-step real-time runs advance in chunks of up to kChunk steps per
-  // gpe_step call (one replayed step graph per step, no host round trip in
-  // between).  A chunk ends before any step at whose start the reference's
+  // gpe_step call (replayed graphs of eight steps and of one, no host round
+  // trip in between).  A chunk ends before any step at whose start the reference's
   // loop does something besides stepping (a save or diagnostic whose test
   // fires, the end of the loop), and at every step after which the norm is
   // needed (eqn 4: a norm record after it or after the next step, whose

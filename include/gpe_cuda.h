@@ -413,7 +413,7 @@ int64_t gpe_state_bytes(const gpe_params* p);
  * double in device memory); the work is queued on `stream` (NULL = the
  * legacy default stream) and the call does not wait for it.
  *
- * Scratch: one partial sum per z-plane in a fixed array inside the library
+ * Scratch: partial sums, at least one per z-plane, in a fixed array inside the library
  * (GPE_NOALLOC_MAX_NZ doubles, 64 KiB), resident on every GPU that loads the
  * library until the process exits.  nz > GPE_NOALLOC_MAX_NZ (or nx, ny,
  * nz < 6, a bad dtype, a NULL pointer) returns GPE_ERR_BADARG and prints the
