@@ -544,10 +544,8 @@ int enqueue_fixed_step(gpe_handle* h, double dr, double di, bool energy, bool no
   return GPE_OK;
 }
 
-// Can stage 6 screen its error ratios in single precision (ck_err_below)?
-bool ck_screen_holds(double dte_r, double dte_i, double inv_adt) {
-  return dte_r >= 0.0 && hypot(dte_r, dte_i) * inv_adt < 1e3;
-}
+// Can stage 6 screen its error ratios (ck_err_below)?  w = (|dt_entry| / |dt|)^2
+bool ck_screen_holds(double dte_r, double w) { return dte_r >= 0.0 && w < 1e100; }
 
 // RKF45 = rkqs (src/solve.f90:158-244) with Cash-Karp stages (248-378)
 int rk45_step(gpe_handle* h, gpe_step_info* io, bool energy, bool norm) {
@@ -585,7 +583,9 @@ int rk45_step(gpe_handle* h, gpe_step_info* io, bool energy, bool norm) {
         a.dte_r = dte_r;
         a.dte_i = dte_i;
         a.inv_adt = 1.0 / hypot(dr, di);
-        if (ck_screen_holds(dte_r, dte_i, a.inv_adt)) a.kout = err_top(h);
+        const double q = hypot(dte_r, dte_i) * a.inv_adt;
+        a.b[0] = q * q;
+        if (ck_screen_holds(dte_r, a.b[0])) a.kout = err_top(h);
         a.want_norm = norm;
       }
       a.want_energy = (m == 0 && energy && first);

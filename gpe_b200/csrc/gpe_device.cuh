@@ -91,7 +91,8 @@ struct alignas(16) StageArgs {
                         // ratio of the launch so far, as ordered bits; null: no screen)
   const void* kin[5];   // Cash-Karp: K_1..K_{m-1}
   double cf_r[2], cf_i[2];  // complex stage coefficients
-  double b[6];              // real Cash-Karp coefficients of this stage
+  double b[6];              // real Cash-Karp coefficients of this stage (stage 6:
+                            // b[0] = (|dt_entry| / |dt|)^2 for the screen of kout)
   double dte_r, dte_i;      // dt at entry of rkqs (psi_scal)
   double inv_adt;           // 1/|dt| of this attempt (psi_scal)
   // stencil constants
@@ -538,24 +539,22 @@ __device__ __forceinline__ double ck_err_ratio(const StageArgs& a, cx<double> pd
   return hypot(er, ei) / hypot(sr, si);
 }
 
-// Is that ratio certainly no larger than top?  Four hypot and a division per
-// site were 34 of stage 6's 344 us (192 x 192 x 384 complex128; 310 so), and only the
-// largest ratio counts, so most sites can be told apart by single-precision
-// square roots of double-precision squares: the estimate is within 1e-6, the
-// margin 1e-4, and anything outside the range where that holds (or NaN) is
-// not "below".  Floats under 1e-38 lose digits: bound is formed without the
-// square of top, whose digits would be gone before a large d2 brought it back,
-// and k2 is off by at most 1.1e-23 in |K1| there, 1.1e-5 of a scale above 1e-15
-// while |dt_entry| / |dt| < 1e3 (and dt_entry is not negative: the host sees to
-// both, ck_screen_holds).
+// Is that ratio certainly no larger than top?  Only the largest ratio counts,
+// and with four hypot and a division at every site stage 6 took 347 us (192 x
+// 192 x 384 complex128; 275 so) and, with empty space around a 192^3 trapped
+// cloud, 195 (161 so).  The square of the scale is at least |psi|^2 + w |K1|^2
+// + 1e-60 (w = (|dt_entry| / |dt|)^2, dt_entry not negative: the host sees to
+// that, ck_screen_holds) and at most three times that, so squares in double
+// precision tell most sites apart, empty ones of a trap among them: a screen
+// in single precision could not, and took 261 us there.  The margin is far
+// above the rounding; a square that underflows is nothing beside 1e-290, and
+// where bound leaves that range (or is NaN) the site is looked at.
 __device__ __forceinline__ bool ck_err_below(const StageArgs& a, cx<double> pd, cx<double> k1, double er, double ei,
                                              double top) {
-  const float e2 = (float)(er * er + ei * ei), p2 = (float)(pd.r * pd.r + pd.i * pd.i);
-  const float k2 = (float)(k1.r * k1.r + k1.i * k1.i);
-  const float fa = sqrtf(k2) * (float)a.inv_adt;
-  const float sr = sqrtf(p2) + (float)a.dte_r * fa, si = (float)a.dte_i * fa;
-  const float d2 = sr * sr + si * si, t = (float)top, bound = t * (t * d2);
-  return e2 * 1.0001f <= bound && bound > 1e-36f && bound < 1e36f && d2 > 1e-30f && d2 < 1e30f;
+  const double e2 = er * er + ei * ei;
+  const double s2 = (pd.r * pd.r + pd.i * pd.i) + (a.b[0] * (k1.r * k1.r + k1.i * k1.i) + 1e-60);
+  const double bound = top * (top * s2);
+  return e2 * 1.000001 <= bound && bound > 1e-290 && bound < 1e290;
 }
 
 // Everything a stage does at the PY interior sites (i, j_q, k) of one thread

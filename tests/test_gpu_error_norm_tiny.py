@@ -34,3 +34,26 @@ def test_error_norm_equals_every_site(gpu, tau, scale):
         out, state = run(rp.replace(tile_zc=march), psi)
         assert out == ref
         np.testing.assert_array_equal(state, sref)
+
+
+# a trapped state with nothing, next to nothing and less than the scale's own
+# 1e-30 around it; attempts that are rejected until dt is far below the one at entry
+@pytest.mark.parametrize("outside", [0.0, 1e-12, 1e-20, 1e-31, 1e-80, 1e-170])
+@pytest.mark.parametrize("storage", ["c128", "c64"])
+@pytest.mark.parametrize("real_time,tau", [(True, 1e-3), (False, 1e-3), (True, 0.2)])
+def test_vacuum(gpu, outside, storage, real_time, tau):
+    if outside and storage == "c64" and outside < 1e-30:
+        outside = 1e-38  # (the storage's own smallest)
+    rp = RunParams(nx=40, ny=21, nz=26, xr=4.875, yr=2.5, zr=3.125, tau=tau, scheme="rk45", eqn_to_solve=4, bcs=2,
+                   order=4, g=1.0, mu=1.0, omx=0.3, omy=0.2, gamma=0.05 if real_time else 0.0, real_time=real_time,
+                   storage=storage)
+    rng = np.random.default_rng(9)
+    psi = 1.0 + 0.1 * (rng.normal(size=(26, 21, 40)) + 1j * rng.normal(size=(26, 21, 40)))
+    full = np.zeros(psi.shape, bool)
+    full[6:18, 5:14, 8:20] = True
+    psi = np.where(full, psi, outside * psi)
+    ref, sref = run(rp, psi)
+    for march in (26, 7):
+        out, state = run(rp.replace(tile_zc=march), psi)
+        assert out == ref
+        np.testing.assert_array_equal(state, sref)
