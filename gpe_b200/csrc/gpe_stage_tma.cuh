@@ -202,11 +202,24 @@ __host__ __device__ constexpr int single_zu() {
                                                                                      : 1;
 }
 
+// May a single-solve stage be launched as a dependent of the one before it (in a
+// step graph)?  The persistent batched kernels are not: they have no free slots
+// to start early in, and lost 8 % with it.
+__host__ __device__ constexpr bool stage_dependent(int k) {
+  return k == K_RK2_1 || k == K_RK2_2 || k == K_RK4_1 || k == K_RK4_2 || k == K_RK4_3 || k == K_RK4_4;
+}
+
+// Does a single-solve stage copy its first planes only after its set-up?  A
+// dependent has to.  The others overlap their copies with the set-up's loads
+// (Cash-Karp stage 2 at 192 x 192 x 384: 206.6 us with late copies, 204.0 so),
+// but Euler's complex64 kernel came out 7 % faster the other way (27.4 and 29.4
+// us at 160^3), complex128 neither.
+__host__ __device__ constexpr bool stage_copies_late(int k, bool dep) { return dep || k == K_EULER; }
+
 // ZU: unroll factor of the z march (the z-queue shifts are renamed across
-// ZU planes); see single_zu.  PDL: the kernel may be launched as a dependent
-// of the previous stage (single-solve kernels; the persistent batched ones
-// have no free slots to start early in, and lost 8 % with it).
-template <class S, class C, int R, int KIND, int TY, int PY, class LY, int ZU = 1, bool PDL = false>
+// ZU planes); see single_zu.  SINGLE: the item is a CTA of a single-solve
+// launch.
+template <class S, class C, int R, int KIND, int TY, int PY, class LY, int ZU = 1, bool SINGLE = false>
 __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a, int bx, int by, int bz,
                                          TmaRing& rg, int* s_abort, double& r_norm, double& r_en,
                                          double& r_err) {
@@ -234,7 +247,7 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
   // Cash-Karp stage 6 of a single solve: the item's largest error ratio so
   // far, shared so that every warp can pass over sites that cannot exceed it
   // (ck_err_below)
-  constexpr bool SCREEN = PDL && KIND == K_CK_6;
+  constexpr bool SCREEN = SINGLE && KIND == K_CK_6;
   __shared__ unsigned long long s_top;
   int issued_s = 0, issued_p = 0;  // meaningful in thread 0 only
   auto issue_stencil = [&](int l) {
@@ -266,6 +279,15 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
     __syncthreads();
   };
 
+  constexpr bool PDL = SINGLE && stage_dependent(KIND), LATE = SINGLE && stage_copies_late(KIND, stage_dependent(KIND));
+  auto issue_first = [&]() {
+    if (tid == 0) {
+      for (int l = 0; l < min(NSS, L); ++l) issue_stencil(l);
+      for (int m = 0; m < min(NPS, M); ++m) issue_pw(m);
+    }
+  };
+  if constexpr (!LATE) issue_first();
+
   // per owned row: grid row, activity, centre offset in a stencil tile
   int jr[PY], cofs[PY];
   bool act[PY];
@@ -286,10 +308,7 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
                    (by * TY + TY - 1 >= g.ny - 1 - R);
 
   if constexpr (PDL) pdl_wait();  // everything above reads host-written tables only
-  if (tid == 0) {
-    for (int l = 0; l < min(NSS, L); ++l) issue_stencil(l);
-    for (int m = 0; m < min(NPS, M); ++m) issue_pw(m);
-  }
+  if constexpr (LATE) issue_first();
 
   auto stile = [&](int l) { return (const S*)(rg.sring + ((SB + l) % NSS) * LY::ST_SLOT); };
   S q[PY][2 * R + 1];  // z queue of each owned row: planes k-R .. k+R
@@ -473,7 +492,7 @@ __device__ __forceinline__ void st_pair(float2* p, float2 v0, float2 v1, bool ac
     *p = v0;
 }
 
-template <class C, int R, int KIND, int TY, int PY, class LY, int ZU = 1, bool PDL = false>
+template <class C, int R, int KIND, int TY, int PY, class LY, int ZU = 1, bool SINGLE = false>
 __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageArgs& a, int bx, int by, int bz,
                                               TmaRing& rg, int* s_abort, double& r_norm, double& r_en,
                                               double& r_err) {
@@ -503,7 +522,7 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
   // Cash-Karp stage 6 of a single solve: the item's largest error ratio so
   // far, shared so that every warp can pass over sites that cannot exceed it
   // (ck_err_below)
-  constexpr bool SCREEN = PDL && KIND == K_CK_6;
+  constexpr bool SCREEN = SINGLE && KIND == K_CK_6;
   __shared__ unsigned long long s_top;
   int issued_s = 0, issued_p = 0;
   auto issue_stencil = [&](int l) {
@@ -533,6 +552,15 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
     __syncthreads();
   };
 
+  constexpr bool PDL = SINGLE && stage_dependent(KIND), LATE = SINGLE && stage_copies_late(KIND, stage_dependent(KIND));
+  auto issue_first = [&]() {
+    if (tid == 0) {
+      for (int l = 0; l < min(NSS, L); ++l) issue_stencil(l);
+      for (int m = 0; m < min(NPS, M); ++m) issue_pw(m);
+    }
+  };
+  if constexpr (!LATE) issue_first();
+
   int jr[PY], cofs[PY], pofs[PY], jq[NS];
   bool act[NS];
   long long o[PY], oq[NS];
@@ -557,10 +585,7 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
                    (by * TY + TY - 1 >= g.ny - 1 - R);
 
   if constexpr (PDL) pdl_wait();  // everything above reads host-written tables only
-  if (tid == 0) {
-    for (int l = 0; l < min(NSS, L); ++l) issue_stencil(l);
-    for (int m = 0; m < min(NPS, M); ++m) issue_pw(m);
-  }
+  if constexpr (LATE) issue_first();
 
   auto stile = [&](int l) { return (const S*)(rg.sring + ((SB + l) % NSS) * LY::ST_SLOT); };
   float4 q[PY][2 * R + 1];  // z queue of each owned row's pair: planes k-R .. k+R
