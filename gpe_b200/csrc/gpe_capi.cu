@@ -206,16 +206,19 @@ int chunk_for(const gpe_handle* h, int per) {
 // CTAs per SM (the Cash-Karp stages with many point-wise inputs hold half as
 // many as the others).
 constexpr int STAGE_MAX_CTAS = 16;  // per SM: 2048 threads in CTAs of 128, the smallest a march has
+int ctas_per_sm(const gpe_handle* h, int kind) {
+  int per = 0;
+  const cudaError_t e = h->cmode == CM_F64   ? stage_tma_occupancy_f64(kind, h->R, h->tma_ty, &per)
+                        : h->cmode == CM_F32 ? stage_tma_occupancy_f32(kind, h->R, h->tma_ty, &per)
+                                             : stage_tma_occupancy_f32x(kind, h->R, h->tma_ty, &per);
+  return e == cudaSuccess ? per : 0;
+}
 int chunk_of(gpe_handle* h, int kind) {
   int& zc = h->zck[kind];
   if (!zc) zc = fixed_chunk(h);
   if (!zc) {
-    int per = 0;
-    const cudaError_t e = h->cmode == CM_F64   ? stage_tma_occupancy_f64(kind, h->R, h->tma_ty, &per)
-                          : h->cmode == CM_F32 ? stage_tma_occupancy_f32(kind, h->R, h->tma_ty, &per)
-                                               : stage_tma_occupancy_f32x(kind, h->R, h->tma_ty, &per);
     // (a kernel that cannot be queried cannot be launched either)
-    zc = chunk_for(h, e == cudaSuccess && per > 0 ? std::min(per, STAGE_MAX_CTAS) : 1);
+    zc = chunk_for(h, std::max(1, std::min(ctas_per_sm(h, kind), STAGE_MAX_CTAS)));
   }
   return zc;
 }
@@ -1027,6 +1030,11 @@ static int ensure_step_graph(gpe_handle* h, int which, double dr, double di) {
   h->step_graph[which] = nullptr;
   h->graph_dt[which][0] = dr;
   h->graph_dt[which][1] = di;
+  // the stages' dependent instances are loaded before the capture, by asking
+  // for their CTAs per SM
+  if (h->use_tma && h->tma_ty != TILE_SITE)
+    for (int k : {K_RK2_1, K_RK2_2, K_RK4_1, K_RK4_2, K_RK4_3, K_RK4_4})
+      if ((k == K_RK2_1 || k == K_RK2_2) == (h->p.scheme == GPE_RK2)) ctas_per_sm(h, k);
   cudaGraph_t g = nullptr;
   CU(h, cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
   h->capturing = true;

@@ -78,16 +78,31 @@ static cudaError_t opt_in_smem(F kernel, uint32_t smem, unsigned long long& done
   return e;
 }
 
-// A null map pointer asks for the kernel's CTAs per SM (in *occ) instead of a launch.
+// Launch one instance of a stage kernel, or with a null map pointer ask for its
+// CTAs per SM (in *occ; the instance is loaded then).
+template <class F>
+static cudaError_t launch_tma_as(F kernel, uint32_t smem, unsigned long long& attr_set, dim3 grid, dim3 block,
+                                 cudaStream_t st, const TmaMaps* m, const StageArgs& a, bool dep, int* occ) {
+  cudaError_t e = opt_in_smem(kernel, smem, attr_set);
+  if (e != cudaSuccess) return e;
+  if (!m) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kernel, block.x * block.y, smem);
+  return launch_stage_kernel(kernel, grid, block, smem, st, dep, *m, a);
+}
+
+// Stages of a step graph (dep) have an instance of their own, which is also the
+// one asked about: long runs replay graphs.
 template <class S, class C, int R, int K, int TY, int PY>
 static cudaError_t launch_tma_one(dim3 grid, cudaStream_t st, const TmaMaps* m, const StageArgs& a, bool dep,
                                   int* occ) {
   using LY = TmaLayout<S, R, StageTraits<K>::NPW, TY>;
+  const dim3 block(32, TY / PY);
+  if constexpr (stage_dependent(K)) {
+    static unsigned long long dep_set = 0;
+    if (dep || !m)
+      return launch_tma_as(k_stage_tma<S, C, R, K, TY, PY, true>, LY::SMEM, dep_set, grid, block, st, m, a, dep, occ);
+  }
   static unsigned long long attr_set = 0;
-  cudaError_t e = opt_in_smem(k_stage_tma<S, C, R, K, TY, PY>, LY::SMEM, attr_set);
-  if (e != cudaSuccess) return e;
-  if (!m) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k_stage_tma<S, C, R, K, TY, PY>, 32 * TY / PY, LY::SMEM);
-  return launch_stage_kernel(k_stage_tma<S, C, R, K, TY, PY>, grid, dim3(32, TY / PY), LY::SMEM, st, dep, *m, a);
+  return launch_tma_as(k_stage_tma<S, C, R, K, TY, PY, false>, LY::SMEM, attr_set, grid, block, st, m, a, false, occ);
 }
 
 template <class S, class C, int R, int TY, int PY>
@@ -121,12 +136,14 @@ template <class C, int R, int K, int TY, int PY>
 static cudaError_t launch_tma_pair_one(dim3 grid, cudaStream_t st, const TmaMaps* m, const StageArgs& a, bool dep,
                                   int* occ) {
   using LY = TmaLayout<float2, R, StageTraits<K>::NPW, TY>;
+  const dim3 block(16, TY / PY);
+  if constexpr (stage_dependent(K)) {
+    static unsigned long long dep_set = 0;
+    if (dep || !m)
+      return launch_tma_as(k_stage_tma_pair<C, R, K, TY, PY, true>, LY::SMEM, dep_set, grid, block, st, m, a, dep, occ);
+  }
   static unsigned long long attr_set = 0;
-  cudaError_t e = opt_in_smem(k_stage_tma_pair<C, R, K, TY, PY>, LY::SMEM, attr_set);
-  if (e != cudaSuccess) return e;
-  if (!m)
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k_stage_tma_pair<C, R, K, TY, PY>, 16 * TY / PY, LY::SMEM);
-  return launch_stage_kernel(k_stage_tma_pair<C, R, K, TY, PY>, grid, dim3(16, TY / PY), LY::SMEM, st, dep, *m, a);
+  return launch_tma_as(k_stage_tma_pair<C, R, K, TY, PY, false>, LY::SMEM, attr_set, grid, block, st, m, a, false, occ);
 }
 
 template <class C, int R, int TY, int PY>

@@ -218,8 +218,9 @@ __host__ __device__ constexpr bool stage_copies_late(int k, bool dep) { return d
 
 // ZU: unroll factor of the z march (the z-queue shifts are renamed across
 // ZU planes); see single_zu.  SINGLE: the item is a CTA of a single-solve
-// launch.
-template <class S, class C, int R, int KIND, int TY, int PY, class LY, int ZU = 1, bool SINGLE = false>
+// launch.  DEP: of one launched as a dependent.
+template <class S, class C, int R, int KIND, int TY, int PY, class LY, int ZU = 1, bool SINGLE = false,
+          bool DEP = false>
 __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a, int bx, int by, int bz,
                                          TmaRing& rg, int* s_abort, double& r_norm, double& r_en,
                                          double& r_err) {
@@ -279,7 +280,7 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
     __syncthreads();
   };
 
-  constexpr bool PDL = SINGLE && stage_dependent(KIND), LATE = SINGLE && stage_copies_late(KIND, stage_dependent(KIND));
+  constexpr bool LATE = SINGLE && stage_copies_late(KIND, DEP);
   auto issue_first = [&]() {
     if (tid == 0) {
       for (int l = 0; l < min(NSS, L); ++l) issue_stencil(l);
@@ -307,7 +308,7 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
   const bool xyg = (bx * TX <= R) || (bx * TX + TX - 1 >= g.nx - 1 - R) || (by * TY <= R) ||
                    (by * TY + TY - 1 >= g.ny - 1 - R);
 
-  if constexpr (PDL) pdl_wait();  // everything above reads host-written tables only
+  if constexpr (DEP) pdl_wait();  // everything above reads host-written tables only
   if constexpr (LATE) issue_first();
 
   auto stile = [&](int l) { return (const S*)(rg.sring + ((SB + l) % NSS) * LY::ST_SLOT); };
@@ -438,7 +439,7 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
     if (++pw_s == NPS) { pw_s = 0; pw_p ^= 1; }
 
     __syncthreads();  // every thread is done with stencil slot lc and point-wise slot m
-    if (PDL && m + 2 >= M) pdl_trigger();
+    if (DEP && m + 2 >= M) pdl_trigger();
     if (*s_abort) {
       drain(ll, m);
       return false;
@@ -456,7 +457,7 @@ __device__ __forceinline__ bool tma_item(const TmaMaps& maps, const StageArgs& a
 }
 
 // Single-solve stage kernel: one work item per CTA (grid = tiles x z-chunks).
-template <class S, class C, int R, int KIND, int TY, int PY>
+template <class S, class C, int R, int KIND, int TY, int PY, bool DEP>
 __global__ void __launch_bounds__(32 * TY / PY) k_stage_tma(const __grid_constant__ TmaMaps maps,
                                                            const StageArgs a) {
   using LY = TmaLayout<S, R, StageTraits<KIND>::NPW, TY>;
@@ -464,7 +465,7 @@ __global__ void __launch_bounds__(32 * TY / PY) k_stage_tma(const __grid_constan
   __shared__ int s_abort;
   TmaRing rg = tma_ring_setup<LY>(smem_raw, &s_abort);
   double r_norm = 0.0, r_en = 0.0, r_err = 0.0;
-  if (!tma_item<S, C, R, KIND, TY, PY, LY, single_zu<S, KIND>(), true>(maps, a, blockIdx.x, blockIdx.y, blockIdx.z, rg,
+  if (!tma_item<S, C, R, KIND, TY, PY, LY, single_zu<S, KIND>(), true, DEP>(maps, a, blockIdx.x, blockIdx.y, blockIdx.z, rg,
                                                                   &s_abort, r_norm,
                                            r_en, r_err))
     return;
@@ -492,7 +493,7 @@ __device__ __forceinline__ void st_pair(float2* p, float2 v0, float2 v1, bool ac
     *p = v0;
 }
 
-template <class C, int R, int KIND, int TY, int PY, class LY, int ZU = 1, bool SINGLE = false>
+template <class C, int R, int KIND, int TY, int PY, class LY, int ZU = 1, bool SINGLE = false, bool DEP = false>
 __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageArgs& a, int bx, int by, int bz,
                                               TmaRing& rg, int* s_abort, double& r_norm, double& r_en,
                                               double& r_err) {
@@ -552,7 +553,7 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
     __syncthreads();
   };
 
-  constexpr bool PDL = SINGLE && stage_dependent(KIND), LATE = SINGLE && stage_copies_late(KIND, stage_dependent(KIND));
+  constexpr bool LATE = SINGLE && stage_copies_late(KIND, DEP);
   auto issue_first = [&]() {
     if (tid == 0) {
       for (int l = 0; l < min(NSS, L); ++l) issue_stencil(l);
@@ -584,7 +585,7 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
   const bool xyg = (bx * TX <= R) || (bx * TX + TX - 1 >= g.nx - 1 - R) || (by * TY <= R) ||
                    (by * TY + TY - 1 >= g.ny - 1 - R);
 
-  if constexpr (PDL) pdl_wait();  // everything above reads host-written tables only
+  if constexpr (DEP) pdl_wait();  // everything above reads host-written tables only
   if constexpr (LATE) issue_first();
 
   auto stile = [&](int l) { return (const S*)(rg.sring + ((SB + l) % NSS) * LY::ST_SLOT); };
@@ -743,7 +744,7 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
     if (++pw_s == NPS) { pw_s = 0; pw_p ^= 1; }
 
     __syncthreads();
-    if (PDL && m + 2 >= M) pdl_trigger();
+    if (DEP && m + 2 >= M) pdl_trigger();
     if (*s_abort) {
       drain(ll, m);
       return false;
@@ -762,7 +763,7 @@ __device__ __forceinline__ bool tma_item_pair(const TmaMaps& maps, const StageAr
 
 // Single-solve stage kernel with two x-adjacent sites per thread
 // (complex64 storage): one work item per CTA, 16 x TY/PY threads.
-template <class C, int R, int KIND, int TY, int PY>
+template <class C, int R, int KIND, int TY, int PY, bool DEP>
 __global__ void __launch_bounds__(16 * TY / PY) k_stage_tma_pair(const __grid_constant__ TmaMaps maps,
                                                                 const StageArgs a) {
   using LY = TmaLayout<float2, R, StageTraits<KIND>::NPW, TY>;
@@ -770,7 +771,7 @@ __global__ void __launch_bounds__(16 * TY / PY) k_stage_tma_pair(const __grid_co
   __shared__ int s_abort;
   TmaRing rg = tma_ring_setup<LY>(smem_raw, &s_abort);
   double r_norm = 0.0, r_en = 0.0, r_err = 0.0;
-  if (!tma_item_pair<C, R, KIND, TY, PY, LY, single_zu<float2, KIND>(), true>(maps, a, blockIdx.x, blockIdx.y, blockIdx.z,
+  if (!tma_item_pair<C, R, KIND, TY, PY, LY, single_zu<float2, KIND>(), true, DEP>(maps, a, blockIdx.x, blockIdx.y, blockIdx.z,
                                                                        rg, &s_abort, r_norm,
                                              r_en, r_err))
     return;
