@@ -21,7 +21,7 @@ constexpr int ROW_GRID = 148 * 8;
 // faster by rows there already.  Each has an instantiation for either (SITES):
 // one with both loops holds fewer threads.
 constexpr int SHORT_ROW = 32, SHORT_PACK = 40;
-// is a row shorter than a warp, or (up to most sites) little longer?
+// is a row shorter than a warp, or a little longer (less than `most` sites)?
 inline bool leaves_lanes(const Geom& g, int most) { return g.nx < most && g.nx != 32; }
 inline bool short_rows(const Geom& g) { return g.nx < SHORT_ROW; }
 

@@ -334,7 +334,10 @@ cudaError_t fft_condensed(const gpe_params& p, const Geom& g, int esz, const voi
   if (cufftSetStream(plan, st) != CUFFT_SUCCESS) return cudaErrorUnknown;
   if (cufftExecZ2Z(plan, (cufftDoubleComplex*)buf, (cufftDoubleComplex*)buf, CUFFT_FORWARD) != CUFFT_SUCCESS)
     return cudaErrorUnknown;
-  const auto spectrum = short_rows(g) ? k_spectrum<true> : k_spectrum<false>;
+  // (folded, a row of 16 still keeps the other lanes' cost below an extra pass:
+  // 26 x 37 x 85 with spectra 117 us folded, 125 with the pass; without spectra
+  // 6 x 1000 x 1000 465 folded, 303 by sites, 16 x 700 x 700 519 folded)
+  const auto spectrum = g.nx < 16 ? k_spectrum<true> : k_spectrum<false>;
   const size_t shm = (size_t)(FFT_THREADS / 32) * nbins * sizeof(double);
   if (shm > 48 * 1024) {
     e = cudaFuncSetAttribute(spectrum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
